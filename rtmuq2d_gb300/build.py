@@ -25,7 +25,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + IN
               "-I" + CSRC, "--expt-relaxed-constexpr"]
 CC_FLAGS = ["-O2", "-fPIC", "-ffp-contract=off", "-std=gnu99", "-I" + INCLUDE]
 
-CU_SOURCES = ["rtm_kernels.cu", "rtm_engine.cu"]
+CU_SOURCES = ["rtm_kernels.cu", "rtm_resident.cu", "rtm_engine.cu"]
 C_SOURCES = ["rtm_host.c", "rtm_zfp.c", "rtm_driver.c"]
 DROPIN_SOURCES = ["rtm_dropin.c"]
 

@@ -29,6 +29,7 @@
 
 #include "rtm_gpu.h"
 #include "rtm_internal.h"
+#include "rtm_partition.h"
 
 namespace rtm {
 
@@ -395,6 +396,18 @@ struct rtm_plan {
     // source-field captures of the next adjoint pass (rtm_plan_capture_source)
     std::vector<int> cap_times;
     void *cap_out = nullptr;
+    // resident passes (k_resident): the blocks of the two passes, and one allocation of their
+    // tables and exchange buffer
+    struct Resident {
+        int nctas = 0, cw = 0;
+        size_t smem = 0;
+        const void *jobs = nullptr;
+        const rtm::ResCta *ctas = nullptr;
+    } res[2];
+    unsigned char *res_base = nullptr;
+    size_t res_bytes = 0, xch_bytes = 0;
+    unsigned long long *xch = nullptr;
+    unsigned res_tag = 1;        // tag of the next launch's first step
 
     template <typename T> T *at(size_t off) { return reinterpret_cast<T *>(base + off); }
 
@@ -441,6 +454,8 @@ static int make_maps(rtm_plan *P)
     return make_plain_map(&P->tm_c, P->base + P->L.coef, P->g, P->es);
 }
 
+static int resident_setup(rtm_plan *P);
+
 static int plan_alloc(const rtm_params &p, rtm_plan **out, bool batched = false)
 {
     RTM_TRY(check_params(p));
@@ -476,6 +491,7 @@ static int plan_alloc(const rtm_params &p, rtm_plan **out, bool batched = false)
     RTM_CUDA(cudaMemcpyAsync(P->base + P->L.rec, rec.data(), rec.size() * sizeof(int),
                              cudaMemcpyHostToDevice, P->stream));
     RTM_CUDA(cudaMemsetAsync(P->base + P->L.status, 0, 256, P->stream));
+    if (!batched) RTM_TRY(resident_setup(P.get()));
     RTM_CUDA(cudaStreamSynchronize(P->stream));
     *out = P.release();
     return RTM_OK;
@@ -486,6 +502,7 @@ static void plan_free(rtm_plan *P)
     if (!P) return;
     if (P->stream) cudaStreamSynchronize(P->stream);
     if (P->base) cudaFree(P->base);
+    if (P->res_base) cudaFree(P->res_base);
     if (P->h_pinned) cudaFreeHost(P->h_pinned);
     for (cudaEvent_t e : P->ev_pool) cudaEventDestroy(e);
     for (int k = 0; k < 2; ++k) {
@@ -651,6 +668,169 @@ static int run_loop(rtm_plan *P, int which, bool graphable, F issue)
     return RTM_OK;
 }
 
+// ---- resident passes ------------------------------------------------------------------------
+// Whether a plan's passes can run resident (k_resident): the scheme's frame of 4 cells stays zero
+// (no shot or receiver on it), the values are stored at full precision, and no step-kernel tile
+// width was asked for.
+static bool resident_wanted(const rtm_plan *P)
+{
+    const Geom &g = P->g;
+    const rtm_params &p = P->p;
+    if (p.tile_x != 0 || p.precision != RTM_PREC_FP32) return false;
+    auto inside = [&](long long x, int z) { return x >= 4 && x < g.dimx - 4 && z >= 4 && z < g.dimz - 4; };
+    if (!inside(g.xs, g.zs)) return false;
+    if (p.rec_count > 0) {
+        const long long c0 = (long long)g.thl + p.rec_first;
+        if (!inside(c0, g.zrec) || !inside(c0 + (long long)(p.rec_spacing - 1) * (p.rec_count - 1), g.zrec))
+            return false;
+    }
+    return true;
+}
+
+template <typename T>
+static ResJob<T> resident_job(rtm_plan *P, int back)
+{
+    ResJob<T> J;
+    memset(&J, 0, sizeof J);
+    const Geom &g = P->g;
+    J.g = g;
+    const T dx = (T)P->p.dx;
+    J.h1 = (T)1.0f / dx;
+    J.h2 = dx * dx;
+    J.h3 = (T)1.0f / (dx * dx);
+    J.back = back;
+    J.t0 = 0;
+    J.t1 = g.nt;
+    J.storage = P->p.storage;
+    for (int k = 0; k < 2; ++k) { J.u[k] = P->at<T>(P->L.u[k]); J.r[k] = P->at<T>(P->L.r[k]); }
+    J.coef = P->at<T>(P->L.coef);
+    for (int k = 0; k < 4; ++k) { J.psi[k] = P->at<T>(P->L.psi[k]); J.xi[k] = P->at<T>(P->L.xi[k]); }
+    const float *prof = P->at<float>(P->L.prof);
+    const ProfLayout pl = prof_layout(g);
+    for (int k = 0; k < 8; ++k) J.prof[k] = prof + pl.off[k];
+    const int *rec = P->at<int>(P->L.rec);
+    J.rec_last = rec; J.rec_first = rec + g.dimx; J.rec_cnt = rec + 2 * g.dimx;
+    J.wav = P->at<float>(P->L.wav);
+    J.seis_t = P->at<float>(P->L.seis_t);
+    J.img = P->at<double>(P->L.img);
+    J.slf = P->at<double>(P->L.slf);
+    J.store = P->at<T>(P->L.store);
+    J.slot_elems = P->L.slot_elems;
+    return J;
+}
+
+template <typename T>
+static int resident_tables(rtm_plan *P, int sms)
+{
+    ResPart part[2];
+    for (int b = 0; b < 2; ++b) {          // a pass without a partition keeps the per-step kernels
+        const int fields = b == 1 && P->p.storage == RTM_STORE_RING ? 2 : 1;
+        if (!res_partition(P->g, fields, (int)sizeof(T), sms, part[b])) part[b] = ResPart();
+    }
+    if (part[0].ctas.empty() && part[1].ctas.empty()) return RTM_OK;
+    const size_t jb = align_up(sizeof(ResJob<T>), 256);
+    size_t cb[2];
+    for (int b = 0; b < 2; ++b) cb[b] = align_up(part[b].ctas.size() * sizeof(ResCta), 256);
+    P->xch_bytes = std::max(part[0].xch_quads, part[1].xch_quads) * 8 * sizeof(T);
+    const size_t total = 2 * jb + cb[0] + cb[1] + P->xch_bytes;
+    if (cudaMalloc(&P->res_base, total) != cudaSuccess) {      // no room: per-step kernels
+        cudaGetLastError();
+        P->res_base = nullptr;
+        return RTM_OK;
+    }
+    P->res_bytes = total;
+    std::vector<unsigned char> h(2 * jb + cb[0] + cb[1], 0);
+    size_t off = 0;
+    for (int b = 0; b < 2; ++b) {
+        const ResJob<T> J = resident_job<T>(P, b);
+        memcpy(h.data() + off, &J, sizeof J);
+        P->res[b].jobs = P->res_base + off;
+        off += jb;
+        memcpy(h.data() + off, part[b].ctas.data(), part[b].ctas.size() * sizeof(ResCta));
+        P->res[b].ctas = reinterpret_cast<const ResCta *>(P->res_base + off);
+        off += cb[b];
+        P->res[b].smem = part[b].smem;
+        P->res[b].cw = part[b].cw;
+        P->res[b].nctas = (int)part[b].ctas.size();
+    }
+    P->xch = reinterpret_cast<unsigned long long *>(P->res_base + off);
+    RTM_CUDA(cudaMemcpyAsync(P->res_base, h.data(), h.size(), cudaMemcpyHostToDevice, P->stream));
+    RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
+    RTM_CUDA(cudaStreamSynchronize(P->stream));
+    return RTM_OK;
+}
+
+// Sets a plan up for resident passes where they apply.
+static int resident_setup(rtm_plan *P)
+{
+    if (!resident_wanted(P)) return RTM_OK;
+    int dev = 0, sms = 0, coop = 0;
+    RTM_CUDA(cudaGetDevice(&dev));
+    RTM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    RTM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return RTM_OK;
+    return P->es == 8 ? resident_tables<double>(P, sms) : resident_tables<float>(P, sms);
+}
+
+// Whether this pass runs resident: not while the stream is being captured (the per-step launches
+// can be), nor with source-field captures between the steps.
+static bool resident_now(rtm_plan *P, int back)
+{
+    if (P->res[back].nctas == 0 || (back && !P->cap_times.empty())) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(P->stream, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cs == cudaStreamCaptureStatusNone;
+}
+
+// Cooperative launches of one device run one after the other: each holds every SM it uses until
+// its last step, so two in flight could wait for SMs the other holds.  The later one's stream
+// waits for the earlier one's end on the device; the host waits for nothing.
+struct ResGate {
+    std::mutex mu;
+    cudaEvent_t last[64] = {};
+};
+static ResGate g_gate;
+
+template <typename T>
+static int run_resident(rtm_plan *P, int back, T *rec_out)
+{
+    const auto &R = P->res[back];
+    const int nt = P->g.nt;
+    if (P->res_tag > 0xffffffffu - (unsigned)nt - 8u) {          // tags start over
+        RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
+        P->res_tag = 1;
+    }
+    ProfBlock pb{nullptr, nullptr, nt};
+    if (P->prof_every > 0) {
+        pb.e0 = P->next_event();
+        pb.e1 = P->next_event();
+        if (!pb.e0 || !pb.e1) return fail(RTM_ERR_CUDA, "event pool");
+        RTM_CUDA(cudaEventRecord(pb.e0, P->stream));
+    }
+    int dev = 0;
+    RTM_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(RTM_ERR_INVALID, "device ordinal %d out of range", dev);
+    {
+        std::lock_guard<std::mutex> lk(g_gate.mu);
+        cudaEvent_t &ev = g_gate.last[dev];
+        if (!ev) RTM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        else RTM_CUDA(cudaStreamWaitEvent(P->stream, ev, 0));
+        RTM_CUDA(launch_resident<T>(static_cast<const ResJob<T> *>(R.jobs), R.ctas, R.nctas, R.cw, R.smem, P->xch, 0,
+                                    nt, P->res_tag, rec_out, P->at<unsigned>(P->L.status), P->stream));
+        RTM_CUDA(cudaEventRecord(ev, P->stream));
+    }
+    P->res_tag += (unsigned)nt + 2u;
+    P->launches++;
+    if (P->prof_every > 0) {
+        RTM_CUDA(cudaEventRecord(pb.e1, P->stream));
+        P->prof_launch[back].push_back(pb);
+    }
+    return RTM_OK;
+}
+
 // Forward pass: SRC/forward_modeling.c:12-159 on the device.
 template <typename T>
 static int run_forward(rtm_plan *P, const float *d_vel, int vel_pitch, const float *d_wav,
@@ -706,7 +886,8 @@ static int run_forward(rtm_plan *P, const float *d_vel, int vel_pitch, const flo
         }
         return RTM_OK;
     };
-    RTM_TRY(run_loop(P, 0, d_seis_out == nullptr, loop));
+    if (resident_now(P, 0)) RTM_TRY(run_resident<T>(P, 0, g.nrec > 0 ? d_seis_out : nullptr));
+    else RTM_TRY(run_loop(P, 0, d_seis_out == nullptr, loop));
     const int c = g.nt & 1;             // u buffer holding u_nt
     P->cur_u = c;
     P->forward_done = true;
@@ -823,7 +1004,8 @@ static int run_adjoint(rtm_plan *P, const float *d_seis)
         }
         return RTM_OK;
     };
-    RTM_TRY(run_loop(P, 1, P->cap_times.empty(), loop));
+    if (resident_now(P, 1)) RTM_TRY(run_resident<T>(P, 1, nullptr));
+    else RTM_TRY(run_loop(P, 1, P->cap_times.empty(), loop));
     const int c = g.nt & 1;             // r buffer holding the last receiver field
     P->cur_r = c;
     P->forward_done = false;   // the stored source wavefield has been consumed

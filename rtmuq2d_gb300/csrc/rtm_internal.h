@@ -233,6 +233,116 @@ int strip_items_host(const Geom &g, int ring);     // k_bstrip items of one memb
 int strip_blocks_host(const Geom &g);              // its strip-quad blocks (16-bit ring scales)
 int boundary_tiles_host(const Geom &g);            // field tiles touching a CPML strip
 
+// ---- resident passes (rtm_resident.cu) ----------------------------------------------------
+// k_resident keeps a pass's fields on the chip: every CTA owns one block of the grid for many
+// time steps and trades only the cells around it with its neighbours.
+constexpr int kResThreads = 512;
+constexpr int kResPad = 8;            // halo cells around a block's tile (psi of the 4 cells beyond
+                                      // the block needs u another 4 beyond)
+constexpr int kResSmem = 224 * 1024;  // dynamic shared memory a block may use (227 KB less the static part)
+constexpr int kResCols = 12;          // columns a thread owns at most
+constexpr int kResItems = 4;          // halo quads a thread moves in one direction at most
+constexpr int kResTmemWords = 128;    // 32-bit tensor-memory words a thread owns (512 columns / 4)
+
+// One block: own cells [xa, xb) x [za, zb) (z on quad bounds) and its mailboxes.  Sides: 0 left,
+// 1 right (depth in columns), 2 up, 3 down (depth in quads); depth 0: no neighbour.
+struct ResCta {
+    int job;
+    int xa, xb, za, zb;
+    int din[4], dout[4];              // halo depth received from / sent to each side
+    int sx[4];                        // the source field crosses this side (reconstruction)
+    unsigned in_off[4], out_off[4];   // the side's mailbox in the exchange buffer (quads)
+    int in_cap[4], out_cap[4];        // quads of one (field, parity) of it
+};
+
+// One pass of one migration, or a run of its steps.
+template <typename T>
+struct ResJob {
+    Geom g;
+    T h1, h2, h3;
+    int back;                         // 0 forward, 1 backward
+    int t0, t1;                       // steps of the pass
+    int storage;
+    T *u[2], *r[2];
+    const T *coef;
+    T *psi[4], *xi[4];                // left, right, top, bottom: only between the runs of a pass
+    const float *prof[8];             // a_l b_l a_r b_r a_t b_t a_b b_b
+    const int *rec_last, *rec_first, *rec_cnt;
+    const float *wav, *seis_t;
+    T *rec_out;                       // forward: recorded seismogram [irec][nt], or NULL
+    double *img, *slf;
+    T *store;                         // ring / snapshot slots
+    size_t slot_elems;
+};
+
+// Shape of a block's tile, its psi strips and its threads' share.
+struct ResShape {
+    int W, H, HQ;                     // columns, rows, quads per column
+    int K, CW;                        // column chunks (one quad each), columns per chunk at most
+    int SP;                           // row pitch of the field tile (odd number of quads)
+    int field;                        // elements of one field tile
+    int cl0, nl, cr0, nr;             // correction columns of the left / right strip
+    int qt0, ht, qb0, hb;             // first row and height of the top / bottom correction quads
+    int PH, PT, PB;                   // row pitches of the psi tiles
+    int offl, offr, offt, offb;       // psi tiles (elements from the tile base)
+    int total;                        // elements
+    int nslot;                        // tensor-memory quads per column
+    int xslot, zslot;                 // slots of xi (x strips, z strips), or -1
+    int cslot;                        // slot of coef, or -1: read from global memory
+    int ring;                         // ring quads of the block (reconstruction), at most
+};
+__host__ __device__ __forceinline__ int res_odd_quads(int n) { return ((n >> 2) & 1) ? n : n + 4; }
+__host__ __device__ __forceinline__ ResShape res_shape(const Geom &g, int xa, int xb, int za, int zb, int fields,
+                                                        int es)
+{
+    ResShape s;
+    s.W = xb - xa; s.H = zb - za; s.HQ = s.H >> 2;
+    const int kmax = kResThreads / s.HQ;
+    s.K = s.W < kmax ? s.W : kmax;
+    s.CW = s.K > 0 ? (s.W + s.K - 1) / s.K : 1 << 20;
+    s.SP = res_odd_quads(s.H + 2 * kResPad);
+    s.field = (s.W + 2 * kResPad) * s.SP;
+    const int cl1 = xb < g.thl - 4 ? xb : g.thl - 4;
+    s.cl0 = xa; s.nl = cl1 > xa ? cl1 - xa : 0;
+    s.cr0 = xa > g.dimx - g.thr + 4 ? xa : g.dimx - g.thr + 4;
+    s.nr = xb > s.cr0 ? xb - s.cr0 : 0;
+    const int tq = (g.thu - 4 + 3) & ~3, t1 = zb < tq ? zb : tq;
+    s.qt0 = za; s.ht = t1 > za ? t1 - za : 0;
+    const int bq = (g.dimz - g.thd + 4) & ~3;
+    s.qb0 = za > bq ? za : bq;
+    s.hb = zb > s.qb0 ? zb - s.qb0 : 0;
+    s.PH = res_odd_quads(s.H); s.PT = res_odd_quads(s.ht + 8); s.PB = res_odd_quads(s.hb + 8);
+    int o = fields * s.field;
+    s.offl = o; if (s.nl) o += (s.nl + 8) * s.PH;
+    s.offr = o; if (s.nr) o += (s.nr + 8) * s.PH;
+    s.offt = o; if (s.ht) o += s.W * s.PT;
+    s.offb = o; if (s.hb) o += s.W * s.PB;
+    s.total = o;
+    s.ring = 0;
+    if (fields == 2 && xa < g.rx1 + 4 && xb > g.rx0 - 4 && za < g.rz1 + 4 && zb > g.rz0 - 4) {
+        if ((za <= g.rz0 - 4 && g.rz0 - 4 < zb) || (za <= g.rz1 && g.rz1 < zb)) s.ring += 2 * s.W;
+        if (xa < g.rx0 || xb > g.rx1) s.ring += 8 * s.HQ;
+    }
+    s.nslot = fields;
+    s.xslot = s.nl || s.nr ? s.nslot++ : -1;
+    s.zslot = s.ht || s.hb ? s.nslot++ : -1;
+    s.cslot = s.CW * (s.nslot + 1) * es <= kResTmemWords ? s.nslot++ : -1;
+    return s;
+}
+// Floats of the block's damping profiles after the tiles (by column, then by row).
+__host__ __device__ __forceinline__ int res_px_floats(const ResShape &s) { return (2 * (s.W + 9) + 3) & ~3; }
+__host__ __device__ __forceinline__ int res_pz_floats(const ResShape &s) { return 2 * (s.H + 2 * kResPad); }
+template <typename T>
+__host__ __device__ __forceinline__ size_t res_smem(const ResShape &s)
+{
+    return ((size_t)s.total + 4 * (size_t)s.ring) * sizeof(T) + sizeof(float) * (size_t)(res_px_floats(s) + res_pz_floats(s));
+}
+// Steps [t0, t1) of every job (of the jobs' own t0, t1 when t1 < 0).  Cooperative: the blocks
+// wait for one another.  cw: the most columns a thread of any block has.
+template <typename T>
+cudaError_t launch_resident(const ResJob<T> *jobs, const ResCta *ctas, int nctas, int cw, size_t smem,
+                            unsigned long long *xch, int t0, int t1, unsigned tag0, T *rec_out,
+                            unsigned *status, cudaStream_t s);
 // ---- launchers (rtm_kernels.cu) --------------------------------------------------------
 // pdl: launch with programmatic stream serialization (overlaps the preceding kernel's tail)
 template <typename T>

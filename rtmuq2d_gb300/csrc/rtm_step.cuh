@@ -26,9 +26,6 @@
 // Consecutive steps chain by programmatic dependent launch: a step's CTAs start while the
 // previous step's last CTAs finish and issue their first tile loads after griddepcontrol.wait.
 
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-
 template <typename T, int WARPS, int BWD>
 struct StepCfg {
     static constexpr int TXC = WARPS * RXC;                       // x columns per tile
@@ -39,68 +36,6 @@ struct StepCfg {
     static constexpr int NS = (sizeof(T) == 4 && !BWD) ? 3 : 2;   // pipeline stages
     static constexpr size_t SMEM = (size_t)NS * STAGE * sizeof(T);
 };
-
-template <typename T>
-__device__ __forceinline__ T add_source(const float *wavelet, int t, T v, T cf)
-{
-    if (sizeof(T) == sizeof(float)) return v + (T)(wavelet[t] * (float)cf);   // float product, as the reference
-    return v + (T)wavelet[t] * cf;
-}
-
-template <typename T>
-__device__ __forceinline__ void image_quad(double *img, double *slf, const T (&s)[4], const T (&r)[4])
-{
-    double2 i0 = reinterpret_cast<double2 *>(img)[0], i1 = reinterpret_cast<double2 *>(img)[1];
-    double2 s0 = reinterpret_cast<double2 *>(slf)[0], s1 = reinterpret_cast<double2 *>(slf)[1];
-    i0.x += (double)s[0] * (double)r[0]; i0.y += (double)s[1] * (double)r[1];
-    i1.x += (double)s[2] * (double)r[2]; i1.y += (double)s[3] * (double)r[3];
-    s0.x += (double)s[0] * (double)s[0]; s0.y += (double)s[1] * (double)s[1];
-    s1.x += (double)s[2] * (double)s[2]; s1.y += (double)s[3] * (double)s[3];
-    reinterpret_cast<double2 *>(img)[0] = i0; reinterpret_cast<double2 *>(img)[1] = i1;
-    reinterpret_cast<double2 *>(slf)[0] = s0; reinterpret_cast<double2 *>(slf)[1] = s1;
-}
-
-// First derivative (times dx) of 4 cells along x from a 9-column window W[k] = f(x-4+k):
-// B4 (f+4 - f-4) + B3 (f+3 - f-3) + B2 (f+2 - f-2) + B1 (f+1 - f-1), the operand order of
-// absorbingBoundaryCondition.c:177-181 (psi) and :198-203 (dpsi).
-template <typename T>
-__device__ __forceinline__ T d1x_w(const T (&W)[9][4], int j)
-{
-    return (T)RTM_B4 * (W[8][j] - W[0][j]) + (T)RTM_B3 * (W[7][j] - W[1][j])
-         + (T)RTM_B2 * (W[6][j] - W[2][j]) + (T)RTM_B1 * (W[5][j] - W[3][j]);
-}
-// The same along z from a 12-value line q (q[4+j] is cell j).
-template <typename T>
-__device__ __forceinline__ T dpsi_z(const T (&q)[12], int j)
-{
-    return (T)RTM_B4 * (q[8 + j] - q[j]) + (T)RTM_B3 * (q[7 + j] - q[1 + j])
-         + (T)RTM_B2 * (q[6 + j] - q[2 + j]) + (T)RTM_B1 * (q[5 + j] - q[3 + j]);
-}
-template <typename T>
-__device__ __forceinline__ T d2x_w(const T (&W)[9][4], int j)
-{
-    return (T)RTM_AC4 * (W[8][j] + W[0][j]) + (T)RTM_AC3 * (W[7][j] + W[1][j])
-         + (T)RTM_AC2 * (W[6][j] + W[2][j]) + (T)RTM_AC1 * (W[5][j] + W[3][j])
-         + (T)RTM_AC0 * W[4][j];
-}
-template <typename T>
-__device__ __forceinline__ T d2z_q(const T (&zz)[12], int j)
-{
-    return (T)RTM_AC4 * (zz[8 + j] + zz[j]) + (T)RTM_AC3 * (zz[7 + j] + zz[1 + j])
-         + (T)RTM_AC2 * (zz[6 + j] + zz[2 + j]) + (T)RTM_AC1 * (zz[5 + j] + zz[3 + j])
-         + (T)RTM_AC0 * zz[4 + j];
-}
-
-// Loads the 12-value z line (zm | centre | zp) of column row `row` of a halo tile.
-template <typename T>
-__device__ __forceinline__ void z_line(const T *tile, int row, int zi, const T (&c)[4], T (&zz)[12])
-{
-    T zm[4], zp[4];
-    ld4(tile + row * SZ + zi - 4, zm);
-    ld4(tile + row * SZ + zi + 4, zp);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { zz[j] = zm[j]; zz[4 + j] = c[j]; zz[8 + j] = zp[j]; }
-}
 
 // The x-strip (left or right) whose psi array holds column x, if any: the left array covers
 // [0, th_left), the right one [dimX-th_right, dimX).  Sets the column's arrays (old psi, new
@@ -128,17 +63,6 @@ __device__ __forceinline__ bool x_strip(const StepArgs<T> &a, int x, const T *&p
         return true;
     }
     return false;
-}
-
-// psi of this step on 4 cells of an x-strip column from the 9-column window of u and the
-// previous psi (absorbingBoundaryCondition.c:177-181, 269-273): psi = b psi + a D1x(u) / dx on
-// z in [4, dimZ-4); the other cells keep their psi.
-template <typename T>
-__device__ __forceinline__ void psi_x_new(const T (&W)[9][4], T (&ps)[4], T ab, T bb, T h1, int zq, int dimz)
-{
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (zq + j >= 4 && zq + j < dimz - 4) ps[j] = bb * ps[j] + ab * d1x_w<T>(W, j) * h1;
 }
 
 // z-strips of a top or bottom tile that touches no x-strip, one column per thread: the band's
@@ -514,21 +438,6 @@ __device__ __forceinline__ void cpml_fused(const StepArgs<T> &a, T *u8, T *sprv,
 // quad-aligned, so a quad is either wholly in a ring band or not: one 16-byte store.  Saving
 // u_t from the halo tile before the CPML pass, rather than u_{t+1} from registers after it
 // with per-cell index arithmetic, took the forward step on 3400 x 700 from 20.0 to 17.9 us.
-// Ring offset of the quad [zq, zq+4) of column x (ring_index of its first cell), or -1 when
-// the quad holds no ring cell.  With quad-aligned region bounds a quad is either wholly in the
-// ring or not, and its 4 cells are consecutive there (ring_save_quad writes the same offsets).
-__device__ __forceinline__ long long ring_quad_offset(const Geom &g, int x, int zq)
-{
-    if (x < g.rx0 - 4 || x >= g.rx1 + 4 || zq < g.rz0 - 4 || zq >= g.rz1 + 4) return -1;
-    if (zq < g.rz0) return (long long)(x - (g.rx0 - 4)) * 4;                              // top band
-    if (zq >= g.rz1) return (long long)4 * g.ring_w + (long long)(x - (g.rx0 - 4)) * 4;   // bottom
-    if (x < g.rx0) return (long long)8 * g.ring_w + (long long)(x - (g.rx0 - 4)) * g.ring_h + (zq - g.rz0);
-    if (x >= g.rx1)
-        return (long long)8 * g.ring_w + (long long)4 * g.ring_h + (long long)(x - g.rx1) * g.ring_h +
-               (zq - g.rz0);
-    return -1;
-}
-
 template <typename T>
 __device__ __forceinline__ void ring_save_quad(const StepArgs<T> &a, const T (&q)[4], int x, int zq)
 {
