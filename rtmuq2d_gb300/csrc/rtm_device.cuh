@@ -312,4 +312,62 @@ __device__ __forceinline__ long long ring_quad_offset(const Geom &g, int x, int 
     return -1;
 }
 
+// The 16-bit storage scale of a block: max |v| over the cells it stores, mapped to target.
+__host__ __device__ __forceinline__ float store_scale_of(float mx, int prec)
+{
+    const float target = prec == 2 ? kFp16Target : kBf16Target;
+    // A block ahead of the wavefront can hold only denormal-size values: clamping keeps the
+    // inverse finite (an infinite inverse would turn 0 into NaN).
+    return fmaxf(mx, 1e-30f) / target;
+}
+
+// Strip quads of one member: every strip column x in [4, thl-4) or [dimx-thr+4, dimx-4)
+// with all its z quads in [4, dimz-4) (nA items), then every column x in [0, dimx) with its
+// top quads (z in [4, thu-4)) and bottom quads (z in [dimz-thd+4, dimz-4)) -- items of strip
+// columns (already covered) or bottom quads outside [4, dimx-4) are skipped (nB items).
+struct CorrShape {
+    int nql, nA, ntq, q0, nbq, nB;
+};
+__host__ __device__ __forceinline__ CorrShape corr_shape(const Geom &g)
+{
+    CorrShape c;
+    c.nql = (g.dimz - 8 + 3) / 4;
+    c.nA = (g.thl - 8 + g.thr - 8) * c.nql;
+    c.ntq = (g.thu - 8 + 3) / 4;
+    c.q0 = (g.dimz - g.thd + 4) & ~3;
+    c.nbq = (g.dimz - 4 - c.q0 + 3) / 4;
+    c.nB = g.dimx * (c.ntq + c.nbq);
+    return c;
+}
+constexpr int kStripBlock = 256;          // strip items per block (and per 16-bit ring scale)
+__host__ __device__ __forceinline__ int round_block(int n)
+{
+    return (n + kStripBlock - 1) / kStripBlock * kStripBlock;
+}
+
+// Item index of quad (x, zq) in the list above (the quad holding a ring cell).
+__device__ __forceinline__ int strip_item(const Geom &g, const CorrShape &cs, int x, int zq)
+{
+    if (x >= 4 && x < g.thl - 4) return (x - 4) * cs.nql + (zq - 4) / 4;
+    if (x >= g.dimx - g.thr + 4 && x < g.dimx - 4)
+        return (g.thl - 8 + x - (g.dimx - g.thr + 4)) * cs.nql + (zq - 4) / 4;
+    const int k = zq < g.thu - 4 ? (zq - 4) / 4 : cs.ntq + (zq - cs.q0) / 4;
+    return cs.nA + x * (cs.ntq + cs.nbq) + k;
+}
+
+// Cell of ring index r (inverse of ring_index).
+__device__ __forceinline__ void ring_cell(const Geom &g, int r, int &x, int &z)
+{
+    const int w4 = g.ring_w * 4;
+    if (r < w4) { x = g.rx0 - 4 + r / 4; z = g.rz0 - 4 + r % 4; return; }
+    r -= w4;
+    if (r < w4) { x = g.rx0 - 4 + r / 4; z = g.rz1 + r % 4; return; }
+    r -= w4;
+    const int h4 = 4 * g.ring_h;
+    if (r < h4) { x = g.rx0 - 4 + r / g.ring_h; z = g.rz0 + r % g.ring_h; return; }
+    r -= h4;
+    x = g.rx1 + r / g.ring_h;
+    z = g.rz0 + r % g.ring_h;
+}
+
 }  // namespace rtm

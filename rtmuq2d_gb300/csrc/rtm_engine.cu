@@ -408,6 +408,8 @@ struct rtm_plan {
     size_t res_bytes = 0, xch_bytes = 0;
     unsigned long long *xch = nullptr;
     unsigned res_tag = 1;        // tag of the next launch's first step
+    float *stage16 = nullptr;    // 16-bit storage: full-precision slots of a run of steps
+    int stage16_slots = 0;
 
     template <typename T> T *at(size_t off) { return reinterpret_cast<T *>(base + off); }
 
@@ -670,13 +672,12 @@ static int run_loop(rtm_plan *P, int which, bool graphable, F issue)
 
 // ---- resident passes ------------------------------------------------------------------------
 // Whether a plan's passes can run resident (k_resident): the scheme's frame of 4 cells stays zero
-// (no shot or receiver on it), the values are stored at full precision, and no step-kernel tile
-// width was asked for.
-static bool resident_wanted(const rtm_plan *P)
+// (no shot or receiver on it), and no step-kernel tile width was asked for.
+static bool resident_wanted(const rtm_plan *P, bool batched = false)
 {
     const Geom &g = P->g;
     const rtm_params &p = P->p;
-    if (p.tile_x != 0 || p.precision != RTM_PREC_FP32) return false;
+    if (p.tile_x != 0 && !batched) return false;
     auto inside = [&](long long x, int z) { return x >= 4 && x < g.dimx - 4 && z >= 4 && z < g.dimz - 4; };
     if (!inside(g.xs, g.zs)) return false;
     if (p.rec_count > 0) {
@@ -732,7 +733,17 @@ static int resident_tables(rtm_plan *P, int sms)
     size_t cb[2];
     for (int b = 0; b < 2; ++b) cb[b] = align_up(part[b].ctas.size() * sizeof(ResCta), 256);
     P->xch_bytes = std::max(part[0].xch_quads, part[1].xch_quads) * 8 * sizeof(T);
-    const size_t total = 2 * jb + cb[0] + cb[1] + P->xch_bytes;
+    P->xch_bytes = align_up(P->xch_bytes, 256);
+    // 16-bit storage: staging for the slots of 64 steps (rings), or for as many snapshots as 32 MB hold
+    size_t stage = 0;
+    if (P->p.precision != RTM_PREC_FP32) {
+        const size_t slot = P->L.slot_elems * sizeof(float);
+        P->stage16_slots = P->p.storage == RTM_STORE_RING
+                               ? std::min(P->L.nslots, 64) + 1
+                               : (int)std::max<size_t>(1, std::min<size_t>((size_t)P->L.nslots, (32u << 20) / slot));
+        stage = slot * P->stage16_slots;
+    }
+    const size_t total = 2 * jb + cb[0] + cb[1] + P->xch_bytes + stage;
     if (cudaMalloc(&P->res_base, total) != cudaSuccess) {      // no room: per-step kernels
         cudaGetLastError();
         P->res_base = nullptr;
@@ -754,6 +765,7 @@ static int resident_tables(rtm_plan *P, int sms)
         P->res[b].nctas = (int)part[b].ctas.size();
     }
     P->xch = reinterpret_cast<unsigned long long *>(P->res_base + off);
+    if (stage) P->stage16 = reinterpret_cast<float *>(P->res_base + off + P->xch_bytes);
     RTM_CUDA(cudaMemcpyAsync(P->res_base, h.data(), h.size(), cudaMemcpyHostToDevice, P->stream));
     RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
     RTM_CUDA(cudaStreamSynchronize(P->stream));
@@ -794,12 +806,31 @@ struct ResGate {
 };
 static ResGate g_gate;
 
+// One cooperative launch on `stream`, after every earlier one on the device.
+template <typename T>
+static int gated_resident(const ResLaunch<T> &L, cudaStream_t stream)
+{
+    int dev = 0;
+    RTM_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(RTM_ERR_INVALID, "device ordinal %d out of range", dev);
+    std::lock_guard<std::mutex> lk(g_gate.mu);
+    cudaEvent_t &ev = g_gate.last[dev];
+    if (!ev) RTM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    else RTM_CUDA(cudaStreamWaitEvent(stream, ev, 0));
+    RTM_CUDA(launch_resident<T>(L, stream));
+    RTM_CUDA(cudaEventRecord(ev, stream));
+    return RTM_OK;
+}
+
+// One pass as resident launches: one, or with 16-bit storage one per staged run of steps, packed after
+// it (forward) or unpacked before it (backward).
 template <typename T>
 static int run_resident(rtm_plan *P, int back, T *rec_out)
 {
     const auto &R = P->res[back];
-    const int nt = P->g.nt;
-    if (P->res_tag > 0xffffffffu - (unsigned)nt - 8u) {          // tags start over
+    const Geom &g = P->g;
+    const int nt = g.nt;
+    if (P->res_tag > 0xffffffffu - 4u * (unsigned)nt - 8u) {     // tags start over
         RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
         P->res_tag = 1;
     }
@@ -810,20 +841,57 @@ static int run_resident(rtm_plan *P, int back, T *rec_out)
         if (!pb.e0 || !pb.e1) return fail(RTM_ERR_CUDA, "event pool");
         RTM_CUDA(cudaEventRecord(pb.e0, P->stream));
     }
-    int dev = 0;
-    RTM_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return fail(RTM_ERR_INVALID, "device ordinal %d out of range", dev);
-    {
-        std::lock_guard<std::mutex> lk(g_gate.mu);
-        cudaEvent_t &ev = g_gate.last[dev];
-        if (!ev) RTM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        else RTM_CUDA(cudaStreamWaitEvent(P->stream, ev, 0));
-        RTM_CUDA(launch_resident<T>(static_cast<const ResJob<T> *>(R.jobs), R.ctas, R.nctas, R.cw, R.smem, P->xch, 0,
-                                    nt, P->res_tag, rec_out, P->at<unsigned>(P->L.status), P->stream));
-        RTM_CUDA(cudaEventRecord(ev, P->stream));
+    ResLaunch<T> L;
+    memset(&L, 0, sizeof L);
+    L.jobs = static_cast<const ResJob<T> *>(R.jobs);
+    L.ctas = R.ctas;
+    L.nctas = R.nctas;
+    L.cw = R.cw;
+    L.smem = R.smem;
+    L.xch = P->xch;
+    L.rec_out = rec_out;
+    L.status = P->at<unsigned>(P->L.status);
+    auto steps = [&](int t0, int t1) -> int {
+        L.t0 = t0;
+        L.t1 = t1;
+        L.tag0 = P->res_tag;
+        P->res_tag += (unsigned)(t1 - t0) + 2u;
+        P->launches++;
+        return gated_resident<T>(L, P->stream);
+    };
+    if (!P->stage16) {
+        RTM_TRY(steps(0, nt));
+    } else {
+        const bool ring = P->p.storage == RTM_STORE_RING;
+        const int run = ring ? P->stage16_slots - 1 : P->stage16_slots * g.slices;
+        Pack16 a;
+        a.g = g;
+        a.stage = P->stage16;
+        a.slot_elems = P->L.slot_elems;
+        a.scales_per_slot = (int)P->L.n_scales_per_slot;
+        a.prec = P->p.precision;
+        for (int t0 = 0; t0 < nt; t0 += run) {
+            const int t1 = std::min(nt, t0 + run);
+            // slots [lo, hi] of the store that steps [t0, t1) write or read; a run's last step also
+            // hands on the ring of the step before it
+            int lo, hi;
+            if (!back) {
+                lo = ring ? t0 + 1 : t0 / g.slices;
+                hi = ring ? std::min(t1, nt - 1) : (t1 - 1) / g.slices;
+            } else {
+                lo = ring ? nt - t1 + 1 : (nt - t1) / g.slices;
+                hi = ring ? nt - std::max(t0 - 1, 2) : (nt - 1 - t0) / g.slices;
+            }
+            a.store = slot_ptr(P, std::max(lo, 0));
+            a.scales = scale_ptr(P, std::max(lo, 0));
+            L.store = reinterpret_cast<T *>(P->stage16) - (ptrdiff_t)lo * (ptrdiff_t)a.slot_elems;
+            const int kind = ring ? kRingTile : kSnapTile;
+            if (back) RTM_CUDA(launch_pack16(kind, false, a, hi - lo + 1, P->stream));
+            RTM_TRY(steps(t0, t1));
+            if (!back) RTM_CUDA(launch_pack16(kind, true, a, hi - lo + 1, P->stream));
+            P->launches += hi >= lo;
+        }
     }
-    P->res_tag += (unsigned)nt + 2u;
-    P->launches++;
     if (P->prof_every > 0) {
         RTM_CUDA(cudaEventRecord(pb.e1, P->stream));
         P->prof_launch[back].push_back(pb);

@@ -242,6 +242,7 @@ constexpr int kResPad = 8;            // halo cells around a block's tile (psi o
 constexpr int kResSmem = 224 * 1024;  // dynamic shared memory a block may use (227 KB less the static part)
 constexpr int kResCols = 12;          // columns a thread owns at most
 constexpr int kResItems = 4;          // halo quads a thread moves in one direction at most
+constexpr int kXchWords = 4;          // 8-byte words of a float quad in the exchange buffer
 constexpr int kResTmemWords = 128;    // 32-bit tensor-memory words a thread owns (512 columns / 4)
 
 // One block: own cells [xa, xb) x [za, zb) (z on quad bounds) and its mailboxes.  Sides: 0 left,
@@ -337,12 +338,36 @@ __host__ __device__ __forceinline__ size_t res_smem(const ResShape &s)
 {
     return ((size_t)s.total + 4 * (size_t)s.ring) * sizeof(T) + sizeof(float) * (size_t)(res_px_floats(s) + res_pz_floats(s));
 }
-// Steps [t0, t1) of every job (of the jobs' own t0, t1 when t1 < 0).  Cooperative: the blocks
-// wait for one another.  cw: the most columns a thread of any block has.
+// Steps [t0, t1) of every job (of the jobs' own t0, t1 when t1 < 0).  Cooperative: the blocks wait
+// for one another.
 template <typename T>
-cudaError_t launch_resident(const ResJob<T> *jobs, const ResCta *ctas, int nctas, int cw, size_t smem,
-                            unsigned long long *xch, int t0, int t1, unsigned tag0, T *rec_out,
-                            unsigned *status, cudaStream_t s);
+struct ResLaunch {
+    const ResJob<T> *jobs;
+    const ResCta *ctas;
+    int nctas, cw;                    // blocks; the most columns a thread of any block has
+    size_t smem;
+    unsigned long long *xch;          // exchange buffer
+    int t0, t1;
+    unsigned tag0;                    // tag of the first step
+    T *rec_out, *store;               // in place of the jobs', unless NULL
+    unsigned *status;
+};
+template <typename T>
+cudaError_t launch_resident(const ResLaunch<T> &L, cudaStream_t s);
+
+// 16-bit storage of resident passes: consecutive slots of the store and of the staging area.
+enum : int { kRingTile = 0, kSnapTile = 1, kRingStrip = 2 };
+struct Pack16 {
+    Geom g;
+    float *stage;                     // full precision, [slot][slot_elems]
+    void *store;
+    float *scales;
+    size_t slot_elems;
+    int scales_per_slot;
+    int prec;
+};
+cudaError_t launch_pack16(int kind, bool pack, const Pack16 &a, int slots, cudaStream_t s);
+
 // ---- launchers (rtm_kernels.cu) --------------------------------------------------------
 // pdl: launch with programmatic stream serialization (overlaps the preceding kernel's tail)
 template <typename T>

@@ -89,15 +89,6 @@ struct MArgs {
     int store_prec;
 };
 
-// The 16-bit storage scale of a block: max |v| over the cells it stores, mapped to target.
-__host__ __device__ __forceinline__ float store_scale_of(float mx, int prec)
-{
-    const float target = prec == 2 ? kFp16Target : kBf16Target;
-    // A block ahead of the wavefront can hold only denormal-size values: clamping keeps the
-    // inverse finite (an infinite inverse would turn 0 into NaN).
-    return fmaxf(mx, 1e-30f) / target;
-}
-
 // The arguments live in shared memory and the tile stores through generic pointers: the
 // __restrict__ qualifiers tell the compiler that those stores never modify the arguments
 // or the stage, so it keeps argument values in registers across them instead of reloading.

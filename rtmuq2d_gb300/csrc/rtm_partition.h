@@ -17,7 +17,7 @@ namespace rtm {
 struct ResPart {
     std::vector<int> xcut, zcut;       // PX + 1, PZ + 1 bounds
     std::vector<ResCta> ctas;          // x-major
-    int cw = 0;                        // the most columns of a chunk
+    int cw = 0;                        // the most columns of a chunk (at least 3: the general kernel is needed)
     size_t smem = 0;                   // dynamic shared memory (bytes)
     size_t xch_quads = 0;              // exchange buffer
     double cost = 0.0;
@@ -96,51 +96,68 @@ inline bool res_partition(const Geom &g, int fields, int es, int sms, ResPart &o
     const int X0 = 4, X1 = g.dimx - 4, Z0 = 4, Z1 = ((g.dimz - 4) + 3) & ~3;
     const double weights[7] = {1.0, 1.3, 1.7, 2.2, 2.8, 3.5, 4.5};
     bool found = false;
-    // the most expensive block of cuts (xc, zc): false when one does not fit, or costs `most`
-    auto measure = [&](const std::vector<int> &xc, const std::vector<int> &zc, bool every, double most, double &cost,
-                       int &cw, size_t &smem) {
-        const int px = (int)xc.size() - 1, pz = (int)zc.size() - 1;
+    // the pieces of one axis: of the plain ones (clear of the strips and of the ring, [s0, s1) and
+    // [r0, r1)) one of each width, and all the others
+    struct Kinds { int n, lo[64], hi[64]; std::vector<int> cut; };
+    auto kinds = [](std::vector<int> cut, int s0, int s1, int r0, int r1, Kinds &k) {
+        k.n = cut.empty() ? 64 : 0;
+        const int p0 = std::max(s0, r0), p1 = std::min(s1, r1);
+        int w[4] = {0, 0, 0, 0}, nw = 0;               // plain widths differ by rounding only
+        for (size_t i = 0; i + 1 < cut.size() && k.n < 64; ++i) {
+            if (cut[i] >= p0 && cut[i + 1] <= p1) {
+                const int width = cut[i + 1] - cut[i];
+                if (width == w[0] || width == w[1] || width == w[2] || width == w[3]) continue;
+                if (nw < 4) w[nw++] = width;
+            }
+            k.lo[k.n] = cut[i];
+            k.hi[k.n++] = cut[i + 1];
+        }
+        k.cut = std::move(cut);
+    };
+    // the most expensive block: false when one does not fit, or costs `most`
+    auto measure = [&](const Kinds &kx, const Kinds &kz, double most, double &cost, int &cw, size_t &smem) {
         cost = 0.0;
         cw = 0;
         smem = 0;
-        for (int i = 0; i < px; ++i) {
-            // the plain columns differ by rounding only: the edges and a few of the rest
-            if (!every && px > 12 && i > 4 && i < px - 5 && i % 7) continue;
-            for (int k = 0; k < pz; ++k) {
-                const ResShape s = res_shape(g, xc[i], xc[i + 1], zc[k], zc[k + 1], fields, es);
+        for (int i = 0; i < kx.n; ++i)
+            for (int k = 0; k < kz.n; ++k) {
+                const ResShape s = res_shape(g, kx.lo[i], kx.hi[i], kz.lo[k], kz.hi[k], fields, es);
                 if (!res_fits(s, es)) return false;
                 cost = std::max(cost, res_cost(s, fields, es));
                 if (cost >= most) return false;
-                cw = std::max(cw, s.CW);
+                // both strips of an axis in one block: the general kernel (NC = 0)
+                cw = std::max(cw, (s.nl && s.nr) || (s.ht && s.hb) ? std::max(3, s.CW) : s.CW);
                 smem = std::max(smem, res_bytes(s, es));
             }
-        }
         if (cw == 2 && es == 4) cost *= 1.2;         // two columns in registers (k_resident's NC) against one
         return cost < most;
     };
     const double cells = (double)(X1 - X0) * (Z1 - Z0);
+    std::vector<Kinds> kx(7), kz(7);
+    int px_of_kx = -1;
     for (int pz = 1; pz <= std::min(sms, std::max(1, (Z1 - Z0) / 8)); ++pz) {
         const int px = std::min(sms / pz, std::max(1, (X1 - X0) / 8));
         if (found && cells / (4.0 * kResThreads * px * pz) * fields * (es == 8 ? 1.0 : 430.0) > out.cost) continue;
-        for (double wz : weights) {
-            const std::vector<int> zc = res_cuts(Z0, Z1, g.thu - 4, g.dimz - g.thd + 4, wz, pz, 4);
-            if (zc.empty()) continue;
-            for (double wx : weights) {
-                const std::vector<int> xc = res_cuts(X0, X1, g.thl - 4, g.dimx - g.thr + 4, wx, px, 1);
-                if (xc.empty()) continue;
-                const double most = found ? out.cost : 1e30;
+        for (int w = 0; w < 7; ++w)
+            kinds(res_cuts(Z0, Z1, g.thu - 4, g.dimz - g.thd + 4, weights[w], pz, 4), g.thu - 4, g.dimz - g.thd + 4, g.rz0,
+                  g.rz1, kz[w]);
+        for (int w = 0; w < 7 && px != px_of_kx; ++w)
+            kinds(res_cuts(X0, X1, g.thl - 4, g.dimx - g.thr + 4, weights[w], px, 1), g.thl - 4, g.dimx - g.thr + 4, g.rx0,
+                  g.rx1, kx[w]);
+        px_of_kx = px;
+        for (const Kinds &z : kz)
+            for (const Kinds &x : kx) {
                 double cost;
                 int cw;
                 size_t smem;
-                if (!measure(xc, zc, false, most, cost, cw, smem) || !measure(xc, zc, true, most, cost, cw, smem)) continue;
+                if (x.n >= 64 || z.n >= 64 || !measure(x, z, found ? out.cost : 1e30, cost, cw, smem)) continue;
                 found = true;
-                out.xcut = xc;
-                out.zcut = zc;
+                out.xcut = x.cut;
+                out.zcut = z.cut;
                 out.cost = cost;
                 out.cw = cw;
                 out.smem = smem;
             }
-        }
     }
     if (!found) return false;
     // mailboxes: one a side with a neighbour, (field, parity) boxes of its depth

@@ -824,7 +824,7 @@ __device__ __forceinline__ void ring_item(const Geom &g, const RingBox &b, int i
 template <typename T, int NC>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_resident(const ResJob<T> *__restrict__ jobs, const ResCta *__restrict__ ctas, unsigned long long *xch, int pt0,
-               int pt1, unsigned tag0, T *rec_out, unsigned *status)
+               int pt1, unsigned tag0, T *rec_out, T *pstore, unsigned *status)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     const Geom &g = J.g;
     const bool back = J.back != 0, ring = J.storage == 1, two = back && ring;
     const int t0 = pt1 < 0 ? J.t0 : pt0, t1 = pt1 < 0 ? J.t1 : pt1;
-    T *rec = J.rec_out ? J.rec_out : rec_out;
+    T *rec = J.rec_out ? J.rec_out : rec_out, *store = pstore ? pstore : J.store;
     const size_t P = (size_t)g.pitch;
     __shared__ ResShape h;
     if (tid == 0) h = res_shape(g, c.xa, c.xb, c.za, c.zb, two ? 2 : 1, (int)sizeof(T));
@@ -882,7 +882,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
     auto s_cur_of = [&](int t) { return ((max(t, 2) - 2) & 1) ? ua : ub; };
 
     // ---- fields, psi and xi on the chip: zero at the first step, else what the last run left
-    for (int i = tid; i < h.total; i += kResThreads) sm[i] = (T)0;
+    const T none[4] = {(T)0, (T)0, (T)0, (T)0};
+    // tiles that load_tile does not fill, and psi
+    for (int i = (t0 > 0 ? (hasS || !two ? h.offl : h.field) : 0) + 4 * tid; i < h.total; i += 4 * kResThreads) st4(sm + i, none);
     for (int i = tid; i < h.W + 9; i += kResThreads) {
         const int x = c.xa - 4 + i;
         float a = 0.0f, b = 0.0f;
@@ -901,14 +903,26 @@ __global__ void __launch_bounds__(kResThreads, 1)
     }
     __syncthreads();
     auto load_tile = [&](const T *f, T *tile) {
-        const int nq = (h.H + 2 * kResPad) >> 2, n = (h.W + 2 * kResPad) * nq;
-        for (int i = tid; i < n; i += kResThreads) {
-            const int k = i / nq, z = c.za - kResPad + 4 * (i - k * nq), x = c.xa - kResPad + k;
-            if (x < 0 || x >= g.dimx || z < 0 || z >= g.pitch) continue;
-            T q[4];
-            ld4(f + (size_t)x * P + z, q);
-            st4(tile + k * h.SP + (z - c.za + kResPad), q);
-        }
+        // a warp takes whole rows of the tile: its lanes along z, up to 4 rows in flight
+        const int nq = h.SP >> 2, rows = h.W + 2 * kResPad, lane = tid & 31;
+        for (int k0 = tid >> 5; k0 < rows; k0 += 4 * (kResThreads / 32))
+            for (int q0 = lane; q0 < nq; q0 += 32) {
+                const int z = c.za - kResPad + 4 * q0;
+                const bool zok = z >= 0 && z < g.pitch && 4 * q0 < h.H + 2 * kResPad;
+                T q[4][4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int k = k0 + r * (kResThreads / 32), x = c.xa - kResPad + k;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) q[r][j] = (T)0;
+                    if (zok && k < rows && x >= 0 && x < g.dimx) ld4(f + (size_t)x * P + z, q[r]);
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int k = k0 + r * (kResThreads / 32);
+                    if (k < rows) st4(tile + k * h.SP + 4 * q0, q[r]);
+                }
+            }
     };
     if (t0 > 0) load_tile(back ? J.r[t0 & 1] : J.u[t0 & 1], su);
     if (hasS) load_tile(J.u[s_cur_of(t0)], ss);
@@ -986,8 +1000,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
         }
     };
     if constexpr (NC == 0) {
-#pragma unroll 1
-        for (int col = 0; col < h.CW; ++col) init_col(col, 0);
+#pragma unroll 4
+        for (int col = 0; col < h.CW; ++col) init_col(col, 0);   // (a column's loads take longer than all the rest)
         tm_wait_st();
     } else {
 #pragma unroll
@@ -1049,7 +1063,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         float seis = 0.0f;
         if (back && my_rec >= 0) seis = J.seis_t[(size_t)(g.nt - 1 - t) * g.nrec + my_rec];
         if (recon && nring > 0) {                           // the ring of u_{nt-t}, for the end of the step
-            const T *slot = J.store + (size_t)(g.nt - t) * J.slot_elems;
+            const T *slot = store + (size_t)(g.nt - t) * J.slot_elems;
             for (int i = tid; i < nring; i += kResThreads) {
                 int x, z;
                 ring_item(g, rb, i, x, z);
@@ -1125,7 +1139,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if (t + 1 < t1) res_send<T>(c, tid, out, recon ? nout : nout0, tag + 1, xch, sm);
         // ---- storage of the forward field, image of the backward ones
         if (!back && ring && t + 1 < g.nt) {            // slot k holds the ring of u_k
-            T *slot = J.store + (size_t)(t + 1) * J.slot_elems;
+            T *slot = store + (size_t)(t + 1) * J.slot_elems;
             for (int i = tid; i < nring; i += kResThreads) {
                 int x, z;
                 ring_item(g, rb, i, x, z);
@@ -1138,7 +1152,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         const bool imaged = img_in == 0;
         img_in = imaged ? g.slices - 1 : img_in - 1;
         if (imaged && int_any && th.own && (back || !ring)) {
-            T *slot = J.store + (size_t)(tau / g.slices) * J.slot_elems;
+            T *slot = store + (size_t)(tau / g.slices) * J.slot_elems;
             const bool zfull = zq >= g.thu && zq + 4 <= g.thu + g.nz;
             const bool zany = zq < g.thu + g.nz && zq + 4 > g.thu;
             for (int col = 0; col < th.len && zany; ++col) {
@@ -1233,7 +1247,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 ld4(ss + (x - c.xa + kResPad) * h.SP + kResPad + (z - c.za), q);
                 st4(sc + (size_t)x * P + z, q);
                 if (t1 > 3) {                            // the step before's ring, from its slot
-                    ld4(J.store + (size_t)(g.nt - t1 + 2) * J.slot_elems + ring_quad_offset(g, x, z), q);
+                    ld4(store + (size_t)(g.nt - t1 + 2) * J.slot_elems + ring_quad_offset(g, x, z), q);
                     st4(sp + (size_t)x * P + z, q);
                 }
             }
@@ -1272,38 +1286,164 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 // ---- launch -----------------------------------------------------------------------------------
 template <typename T, int NC>
-static cudaError_t launch_resident_c(const ResJob<T> *jobs, const ResCta *ctas, int nctas, size_t smem,
-                                     unsigned long long *xch, int t0, int t1, unsigned tag0, T *rec_out, unsigned *status,
-                                     cudaStream_t s)
+static cudaError_t launch_resident_c(const ResLaunch<T> &L, cudaStream_t s)
 {
     static cudaError_t conf = cudaFuncSetAttribute(k_resident<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
     if (conf != cudaSuccess) return conf;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nctas);
+    cfg.gridDim = dim3(L.nctas);
     cfg.blockDim = dim3(kResThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = L.smem;
     cfg.stream = s;
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeCooperative;
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_resident<T, NC>, jobs, ctas, xch, t0, t1, tag0, rec_out, status);
+    return cudaLaunchKernelEx(&cfg, k_resident<T, NC>, L.jobs, L.ctas, L.xch, L.t0, L.t1, L.tag0, L.rec_out, L.store, L.status);
 }
 template <typename T>
-cudaError_t launch_resident(const ResJob<T> *jobs, const ResCta *ctas, int nctas, int cw, size_t smem,
-                            unsigned long long *xch, int t0, int t1, unsigned tag0, T *rec_out, unsigned *status,
-                            cudaStream_t s)
+cudaError_t launch_resident(const ResLaunch<T> &L, cudaStream_t s)
 {
     // registers for a thread's private values while they fit: one quad in double, two in float
-    if (cw <= 1) return launch_resident_c<T, 1>(jobs, ctas, nctas, smem, xch, t0, t1, tag0, rec_out, status, s);
-    if (cw <= 2 && sizeof(T) == 4)
-        return launch_resident_c<T, (sizeof(T) == 4 ? 2 : 1)>(jobs, ctas, nctas, smem, xch, t0, t1, tag0, rec_out, status, s);
-    return launch_resident_c<T, 0>(jobs, ctas, nctas, smem, xch, t0, t1, tag0, rec_out, status, s);
+    if (L.cw <= 1) return launch_resident_c<T, 1>(L, s);
+    if (L.cw <= 2 && sizeof(T) == 4) return launch_resident_c<T, (sizeof(T) == 4 ? 2 : 1)>(L, s);
+    return launch_resident_c<T, 0>(L, s);
 }
-template cudaError_t launch_resident<float>(const ResJob<float> *, const ResCta *, int, int, size_t, unsigned long long *,
-                                            int, int, unsigned, float *, unsigned *, cudaStream_t);
-template cudaError_t launch_resident<double>(const ResJob<double> *, const ResCta *, int, int, size_t,
-                                             unsigned long long *, int, int, unsigned, double *, unsigned *, cudaStream_t);
+template cudaError_t launch_resident<float>(const ResLaunch<float> &, cudaStream_t);
+template cudaError_t launch_resident<double>(const ResLaunch<double> &, cudaStream_t);
+
+// ---- 16-bit storage of a resident pass ---------------------------------------------------------
+// A resident pass reads and writes full-precision slots; with BF16 / FP16 storage they are a staging
+// area of a few slots that these kernels pack into the store after a run of steps, or unpack before
+// one.  Values and scales are those of the per-step kernels: a max-abs scale for each group of a slot's
+// cells -- a tile of the step kernels (kRingTile, kSnapTile) or a strip block of the batched ones
+// (kRingStrip).
+
+// Tile of tile_coords' order that holds cell (x, z).
+__device__ __forceinline__ int tile_at(const Geom &g, int x, int z)
+{
+    const int xt = x / g.tx;
+    int zt = 0;
+    if (z >= g.ztop) zt = g.zbot > 0 && z >= g.zbot ? g.tiles_z - 1 : 1 + (z - g.ztop) / TZ;
+    const int nzb = g.tiles_z > 1 ? 2 : 1;
+    if (zt == 0) return xt * nzb;
+    if (zt == g.tiles_z - 1) return xt * nzb + 1;
+    const int nzi = g.tiles_z - nzb, nxb = g.nxl + (g.tiles_x - g.xr0);
+    int t = g.tiles_x * nzb;
+    if (xt < g.nxl || xt >= g.xr0) return t + (xt < g.nxl ? xt : g.nxl + xt - g.xr0) * nzi + zt - 1;
+    return t + nxb * nzi + (xt - g.nxl) * nzi + zt - 1;
+}
+
+// One group of one slot: blockIdx.x, blockIdx.y.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_pack16(const __grid_constant__ Pack16 a)
+{
+    const Geom &g = a.g;
+    __shared__ float red[8];
+    const float *in = a.stage + (size_t)blockIdx.y * a.slot_elems;
+    unsigned char *out = static_cast<unsigned char *>(a.store) + (size_t)blockIdx.y * a.slot_elems * 2;
+    int x0 = 0, z0 = 0, zend = 0, n = 1;
+    const CorrShape cs = corr_shape(g);
+    if (KIND != kRingStrip) {
+        int xt, zt;
+        tile_coords(g, blockIdx.x, xt, zt);
+        x0 = xt * g.tx; z0 = ztile_origin(g, zt); zend = min(min(ztile_end(g, zt), z0 + TZ), g.dimz);
+        const int x1 = x0 + g.tx;
+        if (KIND == kRingTile) {
+            const bool inside = x0 >= g.rx0 && x1 <= g.rx1 && z0 >= g.rz0 && zend <= g.rz1;
+            if (inside || x0 >= g.rx1 + 4 || x1 <= g.rx0 - 4 || z0 >= g.rz1 + 4 || zend <= g.rz0 - 4) return;
+        } else if (x0 >= g.thl + g.nx || x1 <= g.thl || z0 >= g.thu + g.nz || zend <= g.thu) return;
+        n = (g.tx * (TZ / 4) + 255) / 256;
+    }
+    // offset of the thread's k-th quad in the slot (and its stored cells), or -1
+    auto quad = [&](int k, int &x, int &zq) -> long long {
+        if (KIND == kRingStrip) {
+            int i = blockIdx.x * kStripBlock + threadIdx.x;
+            if (i >= cs.nA + cs.nB) return -1;
+            if (i < cs.nA) {
+                const int c = i / cs.nql;
+                x = c < g.thl - 8 ? 4 + c : g.dimx - g.thr + 4 + (c - (g.thl - 8));
+                zq = 4 + 4 * (i % cs.nql);
+            } else {
+                i -= cs.nA;
+                const int nq = cs.ntq + cs.nbq, q = i % nq;
+                x = i / nq;
+                zq = q < cs.ntq ? 4 + 4 * q : cs.q0 + 4 * (q - cs.ntq);
+                if ((x >= 4 && x < g.thl - 4) || (x >= g.dimx - g.thr + 4 && x < g.dimx - 4)) return -1;
+            }
+            return ring_quad_offset(g, x, zq);
+        }
+        const int i = k * 256 + threadIdx.x;
+        x = x0 + i / (TZ / 4);
+        zq = z0 + 4 * (i % (TZ / 4));
+        if (i >= g.tx * (TZ / 4) || x >= g.dimx || zq >= zend) return -1;
+        if (KIND == kRingTile) return ring_quad_offset(g, x, zq);
+        if (x < g.thl || x >= g.thl + g.nx) return -1;
+        return (long long)(x - g.thl) * g.pitch + zq;
+    };
+    float mx = 0.0f;
+    for (int k = 0; k < n; ++k) {
+        int x = 0, zq = 0;
+        const long long o = quad(k, x, zq);
+        if (o < 0) continue;
+        for (int j = 0; j < 4; ++j)
+            if (KIND != kSnapTile || in_interior(g, x, zq + j)) mx = fmaxf(mx, fabsf(in[o + j]));
+    }
+    mx = block_max<8>(mx, red);
+    const float scale = store_scale_of(mx, a.prec), inv = 1.0f / scale;
+    if (threadIdx.x == 0) a.scales[(size_t)blockIdx.y * a.scales_per_slot + blockIdx.x] = scale;
+    for (int k = 0; k < n; ++k) {
+        int x = 0, zq = 0;
+        const long long o = quad(k, x, zq);
+        if (o < 0) continue;
+        for (int j = 0; j < 4; ++j)
+            if (KIND != kSnapTile || in_interior(g, x, zq + j)) store_put<float>(out, a.prec, (size_t)(o + j), in[o + j], inv);
+    }
+}
+
+// Quads of one slot (blockIdx.y).
+template <int KIND>
+__global__ void __launch_bounds__(256) k_unpack16(const __grid_constant__ Pack16 a)
+{
+    const Geom &g = a.g;
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if ((size_t)4 * i >= a.slot_elems) return;
+    float *out = a.stage + (size_t)blockIdx.y * a.slot_elems + 4 * (size_t)i;
+    const unsigned char *in = static_cast<const unsigned char *>(a.store) + (size_t)blockIdx.y * a.slot_elems * 2;
+    int x, z, group;
+    if (KIND == kSnapTile) {
+        const int pq = g.pitch / 4;
+        x = g.thl + i / pq;
+        z = 4 * (i % pq);
+        if (z + 4 <= g.thu || z >= g.thu + g.nz) return;
+        group = tile_at(g, x, z);
+    } else {
+        ring_cell(g, 4 * i, x, z);
+        group = KIND == kRingTile ? tile_at(g, x, z) : strip_item(g, corr_shape(g), x, z & ~3) / kStripBlock;
+    }
+    const float scale = a.scales[(size_t)blockIdx.y * a.scales_per_slot + group];
+    float q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = store_get<float>(in, a.prec, 4 * (size_t)i + j, scale);
+    st4(out, q);
+}
+
+cudaError_t launch_pack16(int kind, bool pack, const Pack16 &a, int slots, cudaStream_t s)
+{
+    if (slots <= 0) return cudaSuccess;
+    const int groups = kind == kRingStrip ? strip_blocks_host(a.g) : a.g.tiles;
+    const dim3 grid(pack ? groups : (int)((a.slot_elems / 4 + 255) / 256), slots);
+    if (pack) {
+        if (kind == kRingTile) k_pack16<kRingTile><<<grid, 256, 0, s>>>(a);
+        else if (kind == kSnapTile) k_pack16<kSnapTile><<<grid, 256, 0, s>>>(a);
+        else k_pack16<kRingStrip><<<grid, 256, 0, s>>>(a);
+    } else {
+        if (kind == kRingTile) k_unpack16<kRingTile><<<grid, 256, 0, s>>>(a);
+        else if (kind == kSnapTile) k_unpack16<kSnapTile><<<grid, 256, 0, s>>>(a);
+        else k_unpack16<kRingStrip><<<grid, 256, 0, s>>>(a);
+    }
+    return cudaGetLastError();
+}
 
 }  // namespace rtm
