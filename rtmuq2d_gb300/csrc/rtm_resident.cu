@@ -486,35 +486,134 @@ __device__ __forceinline__ void res_leap(const ResJob<T> &J, const ResCta &c, co
     }
 }
 
-// The CPML corrections of one quad of a strip block (absorbingBoundaryCondition.c:191-217, 237-263,
-// 283-310, 330-357), added to its new values v in the reference's order left, top, right, bottom;
-// xx, xz: the quad's xi, updated.  col: the thread's column.  D1(psi) and D2(u) along x are summed a
-// pair of rows at a time, the outermost first, in the operand order of d1x_w / d2x_w.
-template <typename T>
-__device__ __forceinline__ void res_strip_quad(const ResJob<T> &J, const ResCta &c, const ResShape &h, const ResThread &th,
-                                               int col, const T *su, const T *sm, const float *px, const float *pz,
-                                               const T (&cf)[4], T (&xx)[4], T (&xz)[4], T (&v)[4])
+// What stays the same for a thread of a strip block at every step, with NC > 0: its psi quads (xn of
+// the left or right strip, zn of the top or bottom one, at a fixed stride) and where the psi of its own
+// quads lies.  Worked out at every step, the index arithmetic and its chain of shared loads took a
+// third of a small grid's step.  (A block that holds both strips of an axis runs with NC = 0.)
+struct ResFix {
+    int xp, xu, xn, xdp, xdu, xr, xdr, xl;    // psi, u (first of the 9 rows), count, strides; profile; cells before the frame
+    int zp, zu, zn, zdp, zdu, zr, zlo, zhi;   // ..., profile; cells [zlo, zhi) of the quad are updated
+    int sx, sz;                               // psi of the thread's first quad in the x / z strip
+    int xm;                                   // columns of the thread in the x strip (bit u)
+    int slo, shi, sl;                         // cells [slo, shi) of its quads lie in the z strip, sl before the frame
+    bool xfirst;                              // the x correction comes before the z one
+};
+__device__ __forceinline__ void res_fix_init(const Geom &g, const ResCta &c, const ResShape &h, const ResPsi &w,
+                                             const ResThread &th, int tid, ResFix &f)
 {
-    const Geom &g = J.g;
-    const int zq = c.za + 4 * th.q, x = c.xa + th.xk + col, sp = h.SP;
-    const T *up = su + (th.xk + col + kResPad) * sp + kResPad + 4 * th.q;
-    const bool inL = h.nl && x < g.thl - 4, inR = h.nr && x >= g.dimx - g.thr + 4;
-    const bool inT = zq < g.thu - 4, inB = zq + 4 > g.dimz - g.thd + 4;
+    f.xn = f.zn = f.xm = 0;
+    f.sx = f.sz = -1;
+    f.xp = f.xu = f.xdp = f.xdu = f.xr = f.xdr = f.xl = f.zp = f.zu = f.zdp = f.zdu = f.zr = f.zlo = f.zhi = 0;
+    f.slo = f.shi = 0;
+    f.xfirst = true;
+    const int zq = c.za + 4 * th.q;
+    f.sl = g.dimz - 4 - zq;
+    if (h.nl || h.nr) {
+        const int side = h.nl ? 0 : 1, rows = w.rows[side], ks = kResThreads / rows, k = tid / rows, q = tid - k * rows;
+        const int x = w.lo[side] + k;
+        if (k < ks && x < w.hi[side]) {
+            f.xp = (side ? h.offr + (x - h.cr0 + 4) * h.PH : h.offl + (x - h.cl0 + 4) * h.PH) + 4 * q;
+            f.xu = (x - 4 - c.xa + kResPad) * h.SP + kResPad + 4 * q;
+            f.xr = x - c.xa + 4;
+            f.xn = (w.hi[side] - x + ks - 1) / ks;
+            f.xdp = ks * h.PH;
+            f.xdu = ks * h.SP;
+            f.xdr = ks;
+            f.xl = g.dimz - 4 - (c.za + 4 * q);
+        }
+        const int x0 = c.xa + th.xk;
+        for (int u = 0; u < 2; ++u)
+            if (side == 0 ? x0 + u < g.thl - 4 : x0 + u >= g.dimx - g.thr + 4) f.xm |= 1 << u;
+        f.sx = (side ? h.offr + (x0 - h.cr0 + 4) * h.PH : h.offl + (x0 - h.cl0 + 4) * h.PH) + 4 * th.q;
+    }
+    if (h.ht || h.hb) {
+        const int side = h.ht ? 2 : 3, rows = w.rows[side], ks = kResThreads / rows, k = tid / rows, q = tid - k * rows;
+        const int zp = w.lo[side] + 4 * q, pt = side == 2 ? h.PT : h.PB, off = side == 2 ? h.offt : h.offb;
+        const int q0 = (side == 2 ? h.qt0 : h.qb0) - 4;
+        const int zlo = side == 2 ? 4 : g.dimz - g.thd + 4, zhi = side == 2 ? g.thu - 4 : g.dimz - 4;
+        if (k < ks && k < h.W) {
+            f.zp = off + k * pt + (zp - q0);
+            f.zu = (k + kResPad) * h.SP + kResPad + (zp - c.za);
+            f.zr = 2 * (zp - c.za + kResPad);
+            f.zn = (h.W - k + ks - 1) / ks;
+            f.zdp = ks * pt;
+            f.zdu = ks * h.SP;
+            f.zlo = zlo - zp;
+            f.zhi = zhi - zp;
+        }
+        f.slo = zlo - zq;
+        f.shi = zhi - zq;
+        if (f.slo < 4 && f.shi > 0) f.sz = off + th.xk * pt + (zq - q0);
+        else f.slo = f.shi = 0;
+        f.xfirst = h.nl || side == 3;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void res_psi_fix(const ResFix &f, T h1, int sp, const T *su, T *sm, const float *px, const float *pz)
+{
+    {
+        T *pp = sm + f.xp;
+        const T *up = su + f.xu;
+        const float2 *pr = reinterpret_cast<const float2 *>(px) + f.xr;
+#pragma unroll 1
+        for (int i = 0; i < f.xn; ++i, pp += f.xdp, up += f.xdu, pr += f.xdr) {
+            T ps[4], W[9][4];
+            const float2 ab = *pr;
+            ld4(pp, ps);
+#pragma unroll
+            for (int m = 0; m < 9; ++m)
+                if (m != 4) ld4(up + m * sp, W[m]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < f.xl) ps[j] = (T)ab.y * ps[j] + (T)ab.x * d1x_w<T>(W, j) * h1;
+            st4(pp, ps);
+        }
+    }
+    if (f.zn > 0) {
+        T *pp = sm + f.zp;
+        const T *up = su + f.zu;
+        float aa[4], bz[4];
+        ld4(pz + f.zr, aa);
+        ld4(pz + f.zr + 4, bz);
+#pragma unroll 1
+        for (int i = 0; i < f.zn; ++i, pp += f.zdp, up += f.zdu) {
+            T ps[4], zz[12], zm[4], c4[4], zp[4];
+            ld4(pp, ps);
+            ld4(up - 4, zm);
+            ld4(up, c4);
+            ld4(up + 4, zp);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) { zz[m] = zm[m]; zz[4 + m] = c4[m]; zz[8 + m] = zp[m]; }
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (m >= f.zlo && m < f.zhi) ps[m] = (T)bz[m] * ps[m] + (T)aa[m] * dpsi_z<T>(zz, m) * h1;
+            st4(pp, ps);
+        }
+    }
+}
+
+// The CPML corrections of quad u of a thread of a strip block (absorbingBoundaryCondition.c:191-217,
+// 237-263, 283-310, 330-357), added to its new values v in the reference's order left, top, right,
+// bottom; xx, xz: the quad's xi, updated.  up: its u in the tile; psx, psz: its psi.  D1(psi) and D2(u)
+// along x are summed a pair of rows at a time, the outermost first, in the operand order of d1x_w / d2x_w.
+template <typename T>
+__device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h2, T h3, int sp, int ph, const T *up,
+                                               const T *psx, const T *psz, float2 pr, const float *pz, const T (&cf)[4],
+                                               T (&xx)[4], T (&xz)[4], T (&v)[4])
+{
     T dX[4] = {(T)0, (T)0, (T)0, (T)0}, dZ[4] = {(T)0, (T)0, (T)0, (T)0}, uc[4];
+    const bool inX = (f.xm >> u) & 1, inZ = f.sz >= 0;
     ld4(up, uc);
-    if (inL || inR) {
-        const float2 pr = reinterpret_cast<const float2 *>(px)[th.xk + col + 4];
+    if (inX) {
         const T ab = (T)pr.x, bb = (T)pr.y;
-        const int ph = h.PH;
-        const T *ps = sm + (inL ? h.offl + (x - h.cl0 + 4) * ph : h.offr + (x - h.cr0 + 4) * ph) + 4 * th.q;
         const T bk[4] = {(T)RTM_B4, (T)RTM_B3, (T)RTM_B2, (T)RTM_B1};
         const T ak[4] = {(T)RTM_AC4, (T)RTM_AC3, (T)RTM_AC2, (T)RTM_AC1};
         T acc[4], d2[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             T mk[4], pk[4], um[4], uq[4];
-            ld4(ps - (4 - k) * ph, mk);
-            ld4(ps + (4 - k) * ph, pk);
+            ld4(psx - (4 - k) * ph, mk);
+            ld4(psx + (4 - k) * ph, pk);
             ld4(up - (4 - k) * sp, um);
             ld4(up + (4 - k) * sp, uq);
 #pragma unroll
@@ -528,25 +627,22 @@ __device__ __forceinline__ void res_strip_quad(const ResJob<T> &J, const ResCta 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             d2[j] = d2[j] + (T)RTM_AC0 * uc[j];
-            if (zq + j < g.dimz - 4) {
-                const T dp = acc[j] * J.h1;
-                const T xn = bb * xx[j] + ab * (d2[j] * J.h3 + dp);
+            if (j < f.sl) {
+                const T dp = acc[j] * h1;
+                const T xn = bb * xx[j] + ab * (d2[j] * h3 + dp);
                 xx[j] = xn;
-                dX[j] = (cf[j] * J.h2) * (dp + xn);
+                dX[j] = (cf[j] * h2) * (dp + xn);
             }
         }
     }
-    if (inT || inB) {
-        const int zlo = inT ? 4 : g.dimz - g.thd + 4, zhi = inT ? g.thu - 4 : g.dimz - 4;
+    if (inZ) {
         float aa[4], bz[4];
-        ld4(pz + 2 * (4 * th.q + kResPad), aa);
-        ld4(pz + 2 * (4 * th.q + kResPad) + 4, bz);
-        const int kc = min(th.xk + col, h.W - 1);
-        const T *ps = sm + (inT ? h.offt + kc * h.PT + (zq - (h.qt0 - 4)) : h.offb + kc * h.PB + (zq - (h.qb0 - 4)));
+        ld4(pz, aa);
+        ld4(pz + 4, bz);
         T q[12], zz[12], a0[4], a1[4], a2[4];
-        ld4(ps - 4, a0);
-        ld4(ps, a1);
-        ld4(ps + 4, a2);
+        ld4(psz - 4, a0);
+        ld4(psz, a1);
+        ld4(psz + 4, a2);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { q[j] = a0[j]; q[4 + j] = a1[j]; q[8 + j] = a2[j]; }
         ld4(up - 4, a0);
@@ -554,25 +650,23 @@ __device__ __forceinline__ void res_strip_quad(const ResJob<T> &J, const ResCta 
 #pragma unroll
         for (int j = 0; j < 4; ++j) { zz[j] = a0[j]; zz[4 + j] = uc[j]; zz[8 + j] = a2[j]; }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int z = zq + j;
-            if (z >= zlo && z < zhi) {
-                const T dp = dpsi_z<T>(q, j) * J.h1;
-                const T xn = (T)bz[j] * xz[j] + (T)aa[j] * (d2z_q<T>(zz, j) * J.h3 + dp);
+        for (int j = 0; j < 4; ++j)
+            if (j >= f.slo && j < f.shi) {
+                const T dp = dpsi_z<T>(q, j) * h1;
+                const T xn = (T)bz[j] * xz[j] + (T)aa[j] * (d2z_q<T>(zz, j) * h3 + dp);
                 xz[j] = xn;
-                dZ[j] = (cf[j] * J.h2) * (dp + xn);
+                dZ[j] = (cf[j] * h2) * (dp + xn);
             }
-        }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (inL) v[j] = v[j] + dX[j];
-        if (inT) v[j] = v[j] + dZ[j];
-        if (inR) v[j] = v[j] + dX[j];
-        if (inB) v[j] = v[j] + dZ[j];
-        if (zq + j >= g.dimz - 4) v[j] = (T)0;           // the grid's frame stays zero
+        if (inX && f.xfirst) v[j] = v[j] + dX[j];
+        if (inZ) v[j] = v[j] + dZ[j];
+        if (inX && !f.xfirst) v[j] = v[j] + dX[j];
+        if (j >= f.sl) v[j] = (T)0;                      // the grid's frame stays zero
     }
 }
+
 // A product that stays one: the correction is rounded before it is added, as in the other kernels.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
@@ -714,13 +808,19 @@ __device__ __forceinline__ void res_strip_z(const ResJob<T> &J, const ResCta &c,
 // ... of all of a thread's columns.
 template <typename T, int NC>
 __device__ __forceinline__ void res_strips(const ResJob<T> &J, const ResCta &c, const ResShape &h, const ResThread &th,
-                                           const T *su, const T *sm, const float *px, const float *pz, uint32_t tm,
-                                           ResPriv<T, NC> &me)
+                                           const ResFix &f, const T *su, const T *sm, const float *px, const float *pz,
+                                           uint32_t tm, ResPriv<T, NC> &me)
 {
     if constexpr (NC > 0) {
+        const T h1 = J.h1, h2 = J.h2, h3 = J.h3;
+        const int sp = h.SP, ph = h.PH, pt = h.ht ? h.PT : h.PB;
+        const float2 *pr = reinterpret_cast<const float2 *>(px) + th.xk + 4;
+        const T *up = su + (th.xk + kResPad) * sp + kResPad + 4 * th.q;
 #pragma unroll
         for (int u = 0; u < NC; ++u)
-            if (u < h.CW) res_strip_quad<T>(J, c, h, th, u, su, sm, px, pz, me.cf[u], me.xx[u], me.xz[u], me.v[u]);
+            if (u == 0 || u < th.len)
+                res_strip_quad<T>(f, u, h1, h2, h3, sp, ph, up + u * sp, sm + f.sx + u * ph, sm + f.sz + u * pt, pr[u],
+                                  pz + 2 * (4 * th.q + kResPad), me.cf[u], me.xx[u], me.xz[u], me.v[u]);
     } else {
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {                     // left, top; right, bottom
@@ -1042,6 +1142,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
         out[k] = halo_item<false>(h, hout, tid + k * kResThreads);
     }
     const int nin0 = hin.n0, nin = hin.n, nout0 = hout.n0, nout = hout.n;
+    ResFix fix;
+    if constexpr (NC > 0) res_fix_init(g, c, h, wpsi, th, tid, fix);
     int img_in = back ? (g.nt - 1 - t0) % g.slices : (g.slices - t0 % g.slices) % g.slices;   // steps to the next image / snapshot
     const bool int_any = c.xa < g.thl + g.nx && c.xb > g.thl && c.za < g.thu + g.nz && c.zb > g.thu;
     __syncthreads();
@@ -1083,7 +1185,11 @@ __global__ void __launch_bounds__(kResThreads, 1)
             dead = true;
             break;
         }
-        if (strip) res_psi<T>(J, c, h, wpsi, tid, su, sm, px, pz);
+        if constexpr (NC > 0) {
+            if (strip) res_psi_fix<T>(fix, J.h1, h.SP, su, sm, px, pz);
+        } else {
+            if (strip) res_psi<T>(J, c, h, wpsi, tid, su, sm, px, pz);
+        }
         T *own = su + (th.xk + kResPad) * h.SP + kResPad + 4 * th.q;
         auto half = [&](int f) {                              // leapfrog of field f into its tile
             T *tile = sm + f * h.field;
@@ -1093,7 +1199,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
             if (f == 0 && strip) {
                 __syncthreads();                             // psi
-                if (live) res_strips<T, NC>(J, c, h, th, su, sm, px, pz, tm, me);
+                if (live) res_strips<T, NC>(J, c, h, th, fix, su, sm, px, pz, tm, me);
             }
             __syncthreads();
             if (live) {
