@@ -283,7 +283,9 @@ int rtm_server_stats(const rtm_server *server, long long *cell_updates, double *
 /* CUDA-event time (ms) of the batched tile kernel on the second time step of the last
  * rtm_server_step's graph replay, launched without overlapping the kernels around it
  * (steps_per_launch >= 2; 0 otherwise).  For the kernel's roofline; the step itself
- * advances every active member as usual. */
+ * advances every active member as usual.  When no member used the batched kernels (all of
+ * them ran as resident passes), the time of one of the step's resident launches over its
+ * time steps. */
 int rtm_server_kernel_ms(const rtm_server *server, double *tile_kernel_ms);
 /* Tile width of the batched kernel (32 or 16 columns) for p's grid shape, chosen by timing
  * `members` copies of p (nt shortened to `steps`) through a server with each width; later

@@ -23,6 +23,7 @@ struct ServeRequest {
     double t_submit, t_admit, t_done;
     std::vector<float> img, slf;
     long long bytes;
+    bool forced_tile = false;              // the request asked for a batched tile width
 };
 
 }  // namespace rtm
@@ -64,6 +65,27 @@ struct rtm_server {
     cudaEvent_t kev0 = nullptr, kev1 = nullptr;
     bool kernel_sampled = false;
     double kernel_ms_last = 0.0;
+    // resident members (rtm_resident.cu): the host knows their progress, pass 1 or 2 (0: not one) and
+    // step, so their launches need no device state
+    std::vector<int> res_pass, res_step;
+    std::vector<int> res_due;              // steps a member is owed: it gains steps_per_launch a server step
+    struct ResKey {
+        int dimx, dimz, thl, thr, thu, thd, fields, sms;
+        bool operator<(const ResKey &o) const
+        {
+            return std::tie(dimx, dimz, thl, thr, thu, thd, fields, sms) <
+                   std::tie(o.dimx, o.dimz, o.thl, o.thr, o.thu, o.thd, o.fields, o.sms);
+        }
+    };
+    std::map<ResKey, rtm::ResPart> parts;  // blocks per grid shape and SM share (bounded: cleared at 256)
+    rtm::ResJob<float> *d_jobs = nullptr;
+    rtm::ResCta *d_ctas = nullptr;
+    unsigned long long *d_xch = nullptr;   // exchange buffer of the largest launch so far
+    float *d_stage16 = nullptr;            // full-precision slots of the 16-bit members of a launch
+    size_t job_room = 0, cta_room = 0, xch_room = 0, stage16_room = 0;   // elements
+    unsigned res_tag = 1;
+    int res_sampled = 0;                   // steps of the resident launch between kev0 and kev1
+    int sms = 0;
     // host threads decoding ZFP seismograms of submitted requests (rtm_server_submit_zfp)
     std::vector<std::thread> decoders;
     std::deque<rtm::ServeRequest *> to_decode;
@@ -131,7 +153,7 @@ static void rebuild_index(rtm_server *S)
         S->ix.tiles[m] = 0;
         S->ix.nb[m] = 0;
         S->ix.nt[m] = 0;
-        if (S->slot_plan[m]) {
+        if (S->slot_plan[m] && S->res_pass[m] == 0) {
             const rtm_plan *P = S->slot_plan[m];
             const Geom &g = P->g;
             int n[4];
@@ -150,6 +172,245 @@ static void rebuild_index(rtm_server *S)
     S->ix.base2[S->max_members] = b2;
     S->ix.psi_base[S->max_members] = pb;
     S->ix.corr_base[S->max_members] = cb;
+}
+
+// ---- resident members ------------------------------------------------------------------------
+// A server's members run as resident passes where they fit: each rtm_server_step advances every one
+// of them by up to steps_per_launch steps (a launch ends with its member's pass).  Large members take
+// the chip one after the other; small ones share a launch, each with its part of the SMs.
+
+static int res_fields(const rtm_plan *P, int pass) { return pass == 2 && P->p.storage == RTM_STORE_RING ? 2 : 1; }
+
+// Blocks of a member's steps of `pass` on `sms` SMs; NULL when they do not fit.
+static const ResPart *res_part(rtm_server *S, const rtm_plan *P, int pass, int sms)
+{
+    const Geom &g = P->g;
+    const rtm_server::ResKey key{g.dimx, g.dimz, g.thl, g.thr, g.thu, g.thd, res_fields(P, pass), sms};
+    auto it = S->parts.find(key);
+    if (it == S->parts.end()) {
+        ResPart part;
+        if (!res_partition(g, key.fields, 4, sms, part)) part = ResPart();
+        it = S->parts.emplace(key, std::move(part)).first;
+    }
+    return it->second.ctas.empty() ? nullptr : &it->second;
+}
+
+// Whether a request runs resident: no batched tile width asked for, and both passes fit the chip.
+static bool res_member(rtm_server *S, const rtm_plan *P, const ServeRequest *R)
+{
+    if (R->forced_tile || S->sms < 1 || !resident_wanted(P, true)) return false;
+    return res_part(S, P, 1, S->sms) && res_part(S, P, 2, S->sms);
+}
+
+// Device room for `want` elements (grown by a quarter; the stream is idle while it grows).
+template <typename E>
+static int res_room(rtm_server *S, E *&buf, size_t &have, size_t want)
+{
+    if (have >= want) return RTM_OK;
+    RTM_CUDA(cudaStreamSynchronize(S->stream));
+    if (buf) cudaFree(buf);
+    buf = nullptr;
+    have = 0;
+    want += want / 4;
+    if (cudaMalloc(&buf, want * sizeof(E)) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(RTM_ERR_NOMEM, "%zu bytes for the resident members", want * sizeof(E));
+    }
+    have = want;
+    return RTM_OK;
+}
+
+// A member that shares a launch takes about one SM per kResCells cells, in whole shares of the chip so
+// that a few partitions serve every mix: a 400 x 200 grid alone on 152 SMs is bound by its blocks'
+// exchange (3 us a step), and eight of them side by side take little longer than one.
+constexpr double kResCells = 8000.0;
+constexpr int kResMostSteps = 512;        // steps of one launch at most
+
+// One server step of the resident members.  Every one of them is owed steps_per_launch steps; of the
+// launches (members that fit beside one another) a quarter runs, those owed most, each for all the
+// steps it is owed: with four launches or more a member's fields are brought on and off the chip once
+// in four server steps, for the same progress (12 members of 3400 x 700: 3.5 us of 10 a step went into
+// it at 16 steps a launch).
+static int step_resident(rtm_server *S, bool sampled)
+{
+    struct Item {
+        int m, share;                     // slot; it takes sms / share SMs
+        int t0, t1, back;
+        int lo, hi;                       // 16-bit storage: slots its steps write or read
+    };
+    std::vector<Item> items;
+    if (S->parts.size() >= 256) S->parts.clear();
+    for (int m = 0; m < S->max_members; ++m) {
+        const rtm_plan *P = S->slot_plan[m];
+        if (!P || S->res_pass[m] < 1 || S->res_pass[m] > 2) continue;
+        const Geom &g = P->g;
+        Item it;
+        it.m = m;
+        it.back = S->res_pass[m] - 1;
+        it.t0 = S->res_step[m];
+        S->res_due[m] = std::min(S->res_due[m] + S->steps_per_launch, kResMostSteps);
+        it.t1 = std::min(g.nt, it.t0 + S->res_due[m]);
+        it.lo = 0;
+        it.hi = -1;
+        if (P->p.precision != RTM_PREC_FP32) {
+            const int nt = g.nt, sl = g.slices;
+            if (P->p.storage == RTM_STORE_RING) {
+                it.lo = it.back ? nt - it.t1 + 1 : it.t0 + 1;
+                it.hi = it.back ? nt - std::max(it.t0 - 1, 2) : std::min(it.t1, nt - 1);
+            } else {
+                it.lo = (it.back ? nt - it.t1 + sl - 1 : it.t0 + sl - 1) / sl;
+                it.hi = it.back ? (nt - 1 - it.t0) / sl : (it.t1 - 1) / sl;
+            }
+        }
+        const int want = std::max(1, (int)((double)g.dimx * g.dimz / kResCells + 0.999));
+        it.share = std::max(1, std::min(S->sms / want, 16));
+        while (it.share > 1 && !res_part(S, P, it.back + 1, S->sms / it.share)) --it.share;
+        items.push_back(it);
+    }
+    std::stable_sort(items.begin(), items.end(), [](const Item &a, const Item &b) { return a.share < b.share; });
+    auto part_of = [&](const Item &it) { return res_part(S, S->slot_plan[it.m], it.back + 1, S->sms / it.share); };
+
+    // ---- the launches: the largest member left and those that fit beside it
+    std::vector<std::vector<Item>> waves;
+    std::vector<char> taken(items.size(), 0);
+    for (size_t first = 0; first < items.size(); ++first) {
+        if (taken[first]) continue;
+        std::vector<Item> wave;
+        int used = 0;
+        for (size_t i = first; i < items.size(); ++i) {
+            const int need = S->sms / items[i].share;
+            if (taken[i] || used + need > S->sms) continue;
+            taken[i] = 1;
+            used += need;
+            wave.push_back(items[i]);
+        }
+        for (Item &it : wave) {                          // spare SMs to the members in turn
+            const rtm_plan *P = S->slot_plan[it.m];
+            for (int share = 1; share < it.share; ++share) {
+                const int more = S->sms / share - S->sms / it.share;
+                if (used + more > S->sms || !res_part(S, P, it.back + 1, S->sms / share)) continue;
+                used += more;
+                it.share = share;
+                break;
+            }
+        }
+        waves.push_back(std::move(wave));
+    }
+    if (waves.empty()) return RTM_OK;
+    auto due_of = [&](const std::vector<Item> &w) {
+        int d = 0;
+        for (const Item &it : w) d = std::max(d, S->res_due[it.m]);
+        return d;
+    };
+    std::stable_sort(waves.begin(), waves.end(),
+                     [&](const std::vector<Item> &a, const std::vector<Item> &b) { return due_of(a) > due_of(b); });
+    waves.resize((waves.size() + 3) / 4);
+    size_t xch = 0, stage = 0;
+    for (const auto &wave : waves) {
+        size_t wx = 0, ws = 0;
+        for (const Item &it : wave) {
+            wx += part_of(it)->xch_quads;
+            if (it.hi >= it.lo) ws += (size_t)(it.hi - it.lo + 1) * S->slot_plan[it.m]->L.slot_elems;
+        }
+        xch = std::max(xch, wx);
+        stage = std::max(stage, ws);
+    }
+
+    // ---- room, and the tables of all launches in one copy each
+    const size_t words = xch * kXchWords;
+    const bool grown = S->xch_room < words;
+    RTM_TRY(res_room(S, S->d_xch, S->xch_room, words));
+    if (grown || S->res_tag > 0xffffffffu - (unsigned)waves.size() * (kResMostSteps + 2u) - 8u) {
+        RTM_CUDA(cudaMemsetAsync(S->d_xch, 0, S->xch_room * sizeof(unsigned long long), S->stream));
+        S->res_tag = 1;
+    }
+    RTM_TRY(res_room(S, S->d_stage16, S->stage16_room, stage));
+    std::vector<ResJob<float>> jobs;
+    std::vector<ResCta> ctas;
+    std::vector<size_t> wave_ctas;
+    for (const auto &wave : waves) {
+        size_t wx = 0, ws = 0;
+        wave_ctas.push_back(ctas.size());
+        for (const Item &it : wave) {
+            rtm_plan *P = S->slot_plan[it.m];
+            ResJob<float> J = resident_job<float>(P, it.back);
+            J.t0 = it.t0;
+            J.t1 = it.t1;
+            if (P->p.precision != RTM_PREC_FP32) {       // its slots in the staging area, from slot lo on
+                J.store = S->d_stage16 + (ptrdiff_t)ws - (ptrdiff_t)it.lo * (ptrdiff_t)P->L.slot_elems;
+                if (it.hi >= it.lo) ws += (size_t)(it.hi - it.lo + 1) * P->L.slot_elems;
+            }
+            const ResPart *part = part_of(it);
+            for (ResCta c : part->ctas) {
+                c.job = (int)jobs.size();
+                for (int side = 0; side < 4; ++side) { c.in_off[side] += (unsigned)wx; c.out_off[side] += (unsigned)wx; }
+                ctas.push_back(c);
+            }
+            wx += part->xch_quads;
+            jobs.push_back(J);
+        }
+    }
+    wave_ctas.push_back(ctas.size());
+    RTM_TRY(res_room(S, S->d_jobs, S->job_room, jobs.size()));
+    RTM_TRY(res_room(S, S->d_ctas, S->cta_room, ctas.size()));
+    // pageable sources: the copies have read them when they return
+    RTM_CUDA(cudaMemcpyAsync(S->d_jobs, jobs.data(), jobs.size() * sizeof(ResJob<float>), cudaMemcpyHostToDevice, S->stream));
+    RTM_CUDA(cudaMemcpyAsync(S->d_ctas, ctas.data(), ctas.size() * sizeof(ResCta), cudaMemcpyHostToDevice, S->stream));
+
+    for (size_t w = 0; w < waves.size(); ++w) {
+        auto pack = [&](int back) -> int {
+            size_t ws = 0;
+            for (const Item &it : waves[w]) {
+                if (it.hi < it.lo) continue;
+                rtm_plan *P = S->slot_plan[it.m];
+                Pack16 a;
+                a.g = P->g;
+                a.stage = S->d_stage16 + ws;
+                a.store = slot_ptr(P, it.lo);
+                a.scales = scale_ptr(P, it.lo);
+                a.slot_elems = P->L.slot_elems;
+                a.scales_per_slot = (int)P->L.n_scales_per_slot;
+                a.prec = P->p.precision;
+                const int slots = it.hi - it.lo + 1;
+                ws += (size_t)slots * P->L.slot_elems;
+                if (it.back != back) continue;
+                RTM_CUDA(launch_pack16(P->p.storage == RTM_STORE_RING ? kRingStrip : kSnapTile, !back, a, slots, S->stream));
+                S->launches++;
+            }
+            return RTM_OK;
+        };
+        RTM_TRY(pack(1));
+        ResLaunch<float> L;
+        memset(&L, 0, sizeof L);
+        L.jobs = S->d_jobs;
+        L.ctas = S->d_ctas + wave_ctas[w];
+        L.nctas = (int)(wave_ctas[w + 1] - wave_ctas[w]);
+        for (const Item &it : waves[w]) {
+            L.cw = std::max(L.cw, part_of(it)->cw);
+            L.smem = std::max(L.smem, part_of(it)->smem);
+        }
+        L.xch = S->d_xch;
+        L.t1 = -1;
+        L.tag0 = S->res_tag;
+        L.status = S->d_done + 1;
+        S->res_tag += kResMostSteps + 2u;
+        // one launch of a server step without batched members is timed, for rtm_server_kernel_ms
+        const bool sample = w == 0 && sampled;
+        if (sample) RTM_CUDA(cudaEventRecord(S->kev0, S->stream));
+        RTM_TRY(gated_resident<float>(L, S->stream));
+        if (sample) {
+            RTM_CUDA(cudaEventRecord(S->kev1, S->stream));
+            for (const Item &it : waves[w]) S->res_sampled = std::max(S->res_sampled, it.t1 - it.t0);
+        }
+        S->launches++;
+        RTM_TRY(pack(0));
+        for (const Item &it : waves[w]) {
+            S->res_due[it.m] -= it.t1 - it.t0;
+            if (it.t1 == S->slot_plan[it.m]->g.nt) S->res_due[it.m] = 0;     // (the next pass starts afresh)
+            S->res_step[it.m] = it.t1;
+        }
+    }
+    return RTM_OK;
 }
 
 // Uploads one admitted request into slot m on the upload stream: the graph replaying on the
@@ -213,6 +474,9 @@ static int admit(rtm_server *S, int m, ServeRequest *R)
     S->pending.push_back(m);
     S->slot_plan[m] = P;
     S->slot_req[m] = R;
+    S->res_pass[m] = res_member(S, P, R) ? -1 : 0;       // resident from its activation on
+    S->res_step[m] = 0;
+    S->res_due[m] = 0;
     R->t_admit = now_s();
     return RTM_OK;
 }
@@ -227,6 +491,10 @@ static int activate(rtm_server *S)
     RTM_CUDA(cudaEventRecord(S->up_ev, S->up));
     RTM_CUDA(cudaStreamWaitEvent(S->stream, S->up_ev, 0));
     for (int m : S->pending) {
+        if (S->res_pass[m] < 0) {
+            S->res_pass[m] = 1;
+            continue;
+        }
         RTM_CUDA(cudaMemcpyAsync(S->d_mem + m, &S->mem[m], sizeof(BMember<float>), cudaMemcpyHostToDevice,
                                  S->stream));
         RTM_CUDA(cudaMemcpyAsync(S->d_state + m, &kFirstStep, sizeof kFirstStep, cudaMemcpyHostToDevice,
@@ -259,7 +527,7 @@ static int harvest(rtm_server *S, int m)
     unsigned st = 0;
     RTM_CUDA(cudaMemcpyAsync(&st, P->base + P->L.status, sizeof st, cudaMemcpyDeviceToHost, s));
     static const int2 kIdle = {0, 0};
-    RTM_CUDA(cudaMemcpyAsync(S->d_state + m, &kIdle, sizeof kIdle, cudaMemcpyHostToDevice, s));
+    if (S->res_pass[m] == 0) RTM_CUDA(cudaMemcpyAsync(S->d_state + m, &kIdle, sizeof kIdle, cudaMemcpyHostToDevice, s));
     RTM_CUDA(cudaStreamSynchronize(s));
     R->t_done = now_s();
     S->cell_updates_done += 2LL * g.dimx * g.dimz * g.nt;
@@ -367,6 +635,16 @@ static int server_init(rtm_server *S, long long hbm_budget_bytes)
     S->mem.resize(kMaxMembers);
     S->slot_plan.assign(S->max_members, nullptr);
     S->slot_req.assign(S->max_members, nullptr);
+    S->res_pass.assign(S->max_members, 0);
+    S->res_step.assign(S->max_members, 0);
+    S->res_due.assign(S->max_members, 0);
+    {
+        int dev = 0, coop = 0;
+        RTM_CUDA(cudaGetDevice(&dev));
+        RTM_CUDA(cudaDeviceGetAttribute(&S->sms, cudaDevAttrMultiProcessorCount, dev));
+        RTM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        if (!coop) S->sms = 0;
+    }
     memset(&S->ix, 0, sizeof S->ix);
     rebuild_index(S);
     RTM_CUDA(cudaMemcpyAsync(S->d_ix, &S->ix, sizeof S->ix, cudaMemcpyHostToDevice, S->stream));
@@ -409,6 +687,7 @@ static int submit_request(rtm_server *S, const rtm_params *p, const float *veloc
     R->id = S->next_id++;
     R->p = *p;
     R->p.tile_x = q.tile_x;              // the member's tile width in the batched kernel
+    R->forced_tile = p->tile_x != 0;
     const size_t nv = (size_t)(p->th_left + p->nx + p->th_right) * (p->th_up + p->nz + p->th_down);
     R->vel.assign(velocity, velocity + nv);
     if (p->n_wavelet > 0) R->wav.assign(wavelet, wavelet + p->n_wavelet);
@@ -461,6 +740,7 @@ int rtm_server_destroy(rtm_server *S)
     for (auto *R : S->queue) delete R;
     for (auto &kv : S->done) delete kv.second;
     if (S->gexec) cudaGraphExecDestroy(S->gexec);
+    cudaFree(S->d_jobs); cudaFree(S->d_ctas); cudaFree(S->d_xch); cudaFree(S->d_stage16);
     cudaFree(S->d_ix); cudaFree(S->d_mem); cudaFree(S->d_state); cudaFree(S->d_done);
     if (S->h_state) cudaFreeHost(S->h_state);
     for (cudaEvent_t e : {S->ev0, S->ev1, S->kev0, S->kev1, S->up_ev})
@@ -510,11 +790,18 @@ int rtm_server_step(rtm_server *S, int *n_active, int *n_queued)
     int active = 0;
     for (int m = 0; m < S->max_members; ++m) active += S->slot_plan[m] != nullptr;
     active -= (int)S->finished.size();           // members still stepping
+    int batched = 0;
+    for (int m = 0; m < S->max_members; ++m) batched += S->slot_plan[m] != nullptr && S->res_pass[m] == 0;
+    for (int m : S->finished) batched -= S->res_pass[m] == 0;
     if (active > 0) {
         RTM_CUDA(cudaEventRecord(S->ev0, S->stream));
-        RTM_CUDA(cudaGraphLaunch(S->gexec, S->stream));
+        if (batched > 0) {
+            RTM_CUDA(cudaGraphLaunch(S->gexec, S->stream));
+            S->launches += 3LL * S->steps_per_launch;
+        }
+        S->res_sampled = 0;
+        RTM_TRY(step_resident(S, batched == 0));
         RTM_CUDA(cudaEventRecord(S->ev1, S->stream));
-        S->launches += 3LL * S->steps_per_launch;
     }
     // the members that finished in the previous replay, harvested while this one runs
     const bool freed = !S->finished.empty();
@@ -523,11 +810,13 @@ int rtm_server_step(rtm_server *S, int *n_active, int *n_queued)
     // admission in arrival order among the requests whose inputs are ready (a request whose
     // seismogram is still being decoded is passed over; one that does not fit blocks the
     // rest), for as long as the replay runs: one request at least, then while the host time
-    // spent here stays below the previous replay's duration
+    // spent here stays below the previous replay's duration, or kAdmitMs (a small grid's replay
+    // is shorter than one admission, and requests left queued cannot share its launches)
+    constexpr double kAdmitMs = 4.0;
     const double t0 = now_s();
     int admitted = 0;
     for (auto it = S->queue.begin(); it != S->queue.end();) {
-        if (admitted > 0 && (now_s() - t0) * 1e3 > S->last_replay_ms) break;
+        if (admitted > 0 && (now_s() - t0) * 1e3 > std::max(S->last_replay_ms, kAdmitMs)) break;
         ServeRequest *R = *it;
         const int ready = R->ready.load();
         if (ready == 0) { ++it; continue; }
@@ -553,23 +842,31 @@ int rtm_server_step(rtm_server *S, int *n_active, int *n_queued)
     }
     RTM_TRY(activate(S));
     if (active > 0) {
-        RTM_CUDA(cudaMemcpyAsync(S->h_state, S->d_state, sizeof(int2) * S->max_members,
-                                 cudaMemcpyDeviceToHost, S->stream));
+        if (batched > 0)
+            RTM_CUDA(cudaMemcpyAsync(S->h_state, S->d_state, sizeof(int2) * S->max_members,
+                                     cudaMemcpyDeviceToHost, S->stream));
         RTM_CUDA(cudaStreamSynchronize(S->stream));
         float ms = 0.0f;
         RTM_CUDA(cudaEventElapsedTime(&ms, S->ev0, S->ev1));
         S->busy_ms += ms;
         S->last_replay_ms = ms;
-        if (S->kernel_sampled) {
+        if (S->kernel_sampled && (batched > 0 || S->res_sampled > 0)) {
             float kms = 0.0f;
             RTM_CUDA(cudaEventElapsedTime(&kms, S->kev0, S->kev1));
-            S->kernel_ms_last = kms;
+            S->kernel_ms_last = batched > 0 ? kms : kms / S->res_sampled;
         }
         unsigned flags[2] = {0, 0};
         RTM_CUDA(cudaMemcpy(flags, S->d_done, sizeof flags, cudaMemcpyDeviceToHost));
         if (flags[1]) return fail(RTM_ERR_TIMEOUT, "a batched tile load timed out");
-        for (int m = 0; m < S->max_members; ++m)
-            if (S->slot_plan[m] && S->h_state[m].x == 3) S->finished.push_back(m);
+        for (int m = 0; m < S->max_members; ++m) {
+            if (!S->slot_plan[m]) continue;
+            if (S->res_pass[m] == 0) {
+                if (batched > 0 && S->h_state[m].x == 3) S->finished.push_back(m);
+            } else if (S->res_pass[m] < 3 && S->res_step[m] >= S->slot_plan[m]->g.nt) {
+                S->res_step[m] = 0;
+                if (++S->res_pass[m] == 3) S->finished.push_back(m);
+            }
+        }
     }
     // slots freed by this call's harvests leave the work lists before the next replay (an
     // activation above has already rebuilt them)

@@ -131,3 +131,32 @@ def test_capturing_stream_keeps_the_step_kernels(engine):
     torch.cuda.synchronize()
     assert float(want.abs().max()) > 0
     assert float((out - want).norm()) <= 1e-5 * float(want.norm())
+
+
+@pytest.mark.parametrize("steps_per_launch", (16, 7))
+def test_server_members_resident_and_batched_agree(engine, steps_per_launch):
+    """A server's resident members (small ones sharing a launch, 16-bit stores packed by strip block
+    or tile) against the batched kernels (tile_x = 32): within 1e-5, the bar of the batched engine."""
+    from rtmuq2d_gb300 import workloads
+    grids = [(97, 61, (17, 21, 14, 19), 60, 4, {}), (200, 100, (40, 40, 40, 40), 60, 20, dict(precision=1)),
+             (640, 303, (41, 37, 30, 45), 40, 20, {}), (97, 61, (17, 21, 14, 19), 50, 5, dict(storage=0, precision=2)),
+             (300, 133, (60, 12, 13, 64), 49, 7, dict(precision=2)), (301, 150, (33, 20, 25, 40), 60, 4, dict(storage=0)),
+             (1500, 500, (50, 50, 50, 50), 40, 20, dict(precision=1)), (120, 80, (16, 16, 16, 16), 33, 1, {})]
+    requests = []
+    for k, (nx, nz, th, nt, slices, kw) in enumerate(grids):
+        p = workloads.params_tiny(nx=nx, nz=nz, th=16, nt=nt, time_slices=slices)
+        p = p.replace(th_left=th[0], th_right=th[1], th_up=th[2], th_down=th[3], **kw)
+        rng = np.random.default_rng(k)
+        ext = engine.extend_matrix(p, (1600 + 800 * rng.random((nx, nz))).astype(np.float32))
+        requests.append((p, ext, workloads.wavelet_for(p, 60.0),
+                         (0.1 * rng.standard_normal((p.rec_count, nt))).astype(np.float32)))
+    results = []
+    for tile_x in (0, 32):
+        srv = engine.Server(0, max_members=16, steps_per_launch=steps_per_launch)
+        ids = [srv.submit(r[0].replace(tile_x=tile_x), *r[1:]) for r in requests]
+        out = srv.run_all()
+        srv.close()
+        results.append([out[i][:2] for i in ids])
+    for k, (a, b) in enumerate(zip(*results)):
+        for x, y in zip(a, b):
+            assert np.linalg.norm(x.astype(np.float64) - y) <= 1e-5 * np.linalg.norm(y), k
