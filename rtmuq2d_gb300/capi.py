@@ -592,8 +592,8 @@ class Server:
             return None
         # the finished request's size is unknown until polled: use the largest pending one
         n = max(p.nx * p.nz for p in self.params.values())
-        img = np.zeros(n, np.float32)
-        slf = np.zeros(n, np.float32)
+        img = np.empty(n, np.float32)      # untouched pages until a result is written into them
+        slf = np.empty(n, np.float32)
         rid = C.c_longlong()
         times = (C.c_double * 3)()
         st = lib().rtm_server_poll(self.handle, C.byref(rid), _fp(img), _fp(slf), times)
@@ -602,8 +602,11 @@ class Server:
         _check(st)
         p = self.params.pop(rid.value)
         m = p.nx * p.nz
-        return (rid.value, img[:m].reshape(p.nx, p.nz).copy(), slf[:m].reshape(p.nx, p.nz).copy(),
-                tuple(times))
+
+        def fit(a):                        # no copy of a result that fills most of its buffer
+            a = a[:m] if 2 * m > n else a[:m].copy()
+            return a.reshape(p.nx, p.nz)
+        return rid.value, fit(img), fit(slf), tuple(times)
 
     def wait(self, request_id: int):
         """Steps until request_id has finished: (image, self_image, (t_submit, t_admit, t_done))."""
