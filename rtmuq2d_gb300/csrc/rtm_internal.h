@@ -287,9 +287,8 @@ struct ResShape {
     int PH, PT, PB;                   // row pitches of the psi tiles
     int offl, offr, offt, offb;       // psi tiles (elements from the tile base)
     int total;                        // elements
-    int nslot;                        // tensor-memory quads per column
+    int nslot;                        // tensor-memory quads per column (and one of coef from the second on)
     int xslot, zslot;                 // slots of xi (x strips, z strips), or -1
-    int cslot;                        // slot of coef, or -1: read from global memory
     int ring;                         // ring quads of the block (reconstruction), at most
 };
 __host__ __device__ __forceinline__ int res_odd_quads(int n) { return ((n >> 2) & 1) ? n : n + 4; }
@@ -327,7 +326,6 @@ __host__ __device__ __forceinline__ ResShape res_shape(const Geom &g, int xa, in
     s.nslot = fields;
     s.xslot = s.nl || s.nr ? s.nslot++ : -1;
     s.zslot = s.ht || s.hb ? s.nslot++ : -1;
-    s.cslot = s.CW * (s.nslot + 1) * es <= kResTmemWords ? s.nslot++ : -1;
     return s;
 }
 // Floats of the block's damping profiles after the tiles (by column, then by row).

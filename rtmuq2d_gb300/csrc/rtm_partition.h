@@ -45,10 +45,11 @@ inline std::vector<int> res_cuts(int lo, int hi, int s0, int s1, double w, int p
 }
 
 // Time of a block's step in ns, from the phases' times on GB300 (clock64 around them, 400 x 200,
-// 2000 x 600 and 3400 x 700 grids): a column of the leapfrog 330 with coef in tensor memory, 420
-// without, and 100 to swap it into the tile; a column of a top or bottom strip 520, of a left or right
-// one 500 (only the columns in it); psi 550 (left, right) and 350 (top, bottom) a round of the threads
-// over its quads; a halo round 400; the ring 800.
+// 2000 x 600 and 3400 x 700 grids): a column of the leapfrog 330, and 100 to swap it into the tile; a
+// column of a top or bottom strip 520, of a left or right one 500 (only the columns in it); psi 550
+// (left, right) and 350 (top, bottom) a round of the threads over its quads; a halo round 400; the
+// ring 800.  Scaling the strips', psi's, halo's or ring's share by 0.6 to 1.5 gained nothing over nine
+// grids from 400 x 200 to 3400 x 700 (most stayed within 2 %, the worst lost 30 %).
 // Double runs at the FP64 pipe's pace (2 operations a cycle and SM): 20 operations a cell and field
 // and 36 more a strip, and half as long again when a thread's values do not fit its registers.
 inline double res_cost(const ResShape &s, int fields, int es)
@@ -59,7 +60,7 @@ inline double res_cost(const ResShape &s, int fields, int es)
         return (ops / 3.8 + 1500.0) * (s.CW > 1 ? 1.5 : 1.0);
     }
     const int nx = std::max(s.nl, s.nr);
-    double c = s.CW * fields * ((s.cslot >= 0 ? 330.0 : 420.0) + 100.0);
+    double c = s.CW * fields * 430.0;
     if (s.zslot >= 0) c += 520.0 * s.CW;
     if (s.xslot >= 0) c += 500.0 * std::min(s.CW, nx);
     auto rounds = [](int cols, int rows) {
@@ -86,7 +87,8 @@ inline int res_halo_most(const ResShape &s) { return 2 * (8 + 4) * s.HQ + 2 * (2
 inline bool res_fits(const ResShape &s, int es)
 {
     return s.HQ >= 1 && s.HQ <= kResThreads && s.W <= kResThreads && 2 * s.W + 8 * s.HQ <= 2 * kResThreads &&
-           s.CW <= kResCols && s.CW * s.nslot * es <= kResTmemWords && (s.cslot >= 0 || (s.xslot < 0 && s.zslot < 0)) && res_halo_most(s) <= kResItems * kResThreads &&
+           s.CW <= kResCols && (s.CW * s.nslot + s.CW - 1) * es <= kResTmemWords &&
+           res_halo_most(s) <= kResItems * kResThreads &&
            (s.nslot > 1 ? 2 : 1) * s.field < (1 << 17) && res_bytes(s, es) <= (size_t)kResSmem;
 }
 

@@ -267,20 +267,23 @@ __device__ __forceinline__ bool res_recv(const ResCta &c, int tid, const unsigne
     return ok;
 }
 
-// Publishes the first n items that the neighbours need.
-template <typename T>
+// Publishes the first n items that the neighbours need, R a round: their loads are in flight together.
+template <typename T, int R>
 __device__ __forceinline__ void res_send(const ResCta &c, int tid, const unsigned (&out)[kResItems], int n, unsigned tag,
                                          unsigned long long *xch, const T *tile)
 {
     const int par = (int)(tag & 1u);
 #pragma unroll
-    for (int k = 0; k < kResItems; ++k) {
-        if (k > 0 && k * kResThreads >= n) break;
-        if (tid + k * kResThreads < n) {
-            T q[4];
-            ld4(tile + 4 * (out[k] & 0x7fffu), q);
-            x_put<T>(xch + halo_word<T>(c.out_off, c.out_cap, out[k], par), q, tag);
-        }
+    for (int r = 0; r < kResItems; r += R) {
+        if (r > 0 && r * kResThreads >= n) break;
+        T q[R][4];
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (tid + (r + k) * kResThreads < n) ld4(tile + 4 * (out[r + k] & 0x7fffu), q[k]);
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (tid + (r + k) * kResThreads < n)
+                x_put<T>(xch + halo_word<T>(c.out_off, c.out_cap, out[r + k], par), q[k], tag);
     }
 }
 
@@ -331,16 +334,32 @@ __device__ __forceinline__ void res_psi(const ResJob<T> &J, const ResCta &c, con
         T *pp = sm + (side ? h.offr + (x - h.cr0 + 4) * ph : h.offl + (x - h.cl0 + 4) * ph) + 4 * q;
         const T *up = su + (x - 4 - c.xa + kResPad) * sp + kResPad + 4 * q;
         const float2 *pr = reinterpret_cast<const float2 *>(px) + (x - c.xa + 4);
+        // two quads at a time: their loads come before either store
 #pragma unroll 1
-        for (; x < hi; x += ks, pp += ks * ph, up += ks * sp, pr += ks) {
-            T ps[4], W[9][4];
-            const float2 ab = *pr;
-            ld4(pp, ps);
+        for (; x < hi; x += 2 * ks, pp += 2 * ks * ph, up += 2 * ks * sp, pr += 2 * ks) {
+            const bool two = x + ks < hi;
+            T ps[2][4], d1[2][4];
+            float2 ab[2];
 #pragma unroll
-            for (int m = 0; m < 9; ++m)
-                if (m != 4) ld4(up + m * sp, W[m]);
-            psi_x_new<T>(W, ps, (T)ab.x, (T)ab.y, h1, zq, dimz);
-            st4(pp, ps);
+            for (int u = 0; u < 2; ++u) {
+                const int o = u && two ? ks : 0;
+                ab[u] = pr[o];
+                ld4(pp + o * ph, ps[u]);
+                T W[9][4];
+#pragma unroll
+                for (int m = 0; m < 9; ++m)
+                    if (m != 4) ld4(up + (o + m) * sp, W[m]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d1[u][j] = d1x_w<T>(W, j);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u && !two) break;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (zq + j < dimz - 4) ps[u][j] = (T)ab[u].y * ps[u][j] + (T)ab[u].x * d1[u][j] * h1;
+                st4(pp + (u ? ks * ph : 0), ps[u]);
+            }
         }
     }
 #pragma unroll 1
@@ -357,20 +376,32 @@ __device__ __forceinline__ void res_psi(const ResJob<T> &J, const ResCta &c, con
         ld4(pz + 2 * (zq - c.za + kResPad), aa);
         ld4(pz + 2 * (zq - c.za + kResPad) + 4, bz);
 #pragma unroll 1
-        for (int x = k; x < W; x += ks, pp += ks * pt, up += ks * sp) {
-            T ps[4], zz[12], zm[4], c4[4], zp[4];
-            ld4(pp, ps);
-            ld4(up - 4, zm);
-            ld4(up, c4);
-            ld4(up + 4, zp);
+        for (int x = k; x < W; x += 2 * ks, pp += 2 * ks * pt, up += 2 * ks * sp) {
+            const bool two = x + ks < W;
+            T ps[2][4], d1[2][4];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) { zz[m] = zm[m]; zz[4 + m] = c4[m]; zz[8 + m] = zp[m]; }
+            for (int u = 0; u < 2; ++u) {
+                const int o = u && two ? ks : 0;
+                T zz[12], zm[4], c4[4], zp[4];
+                ld4(pp + o * pt, ps[u]);
+                ld4(up + o * sp - 4, zm);
+                ld4(up + o * sp, c4);
+                ld4(up + o * sp + 4, zp);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int z = zq + m;
-                if (z >= zlo && z < zhi) ps[m] = (T)bz[m] * ps[m] + (T)aa[m] * dpsi_z<T>(zz, m) * h1;
+                for (int m = 0; m < 4; ++m) { zz[m] = zm[m]; zz[4 + m] = c4[m]; zz[8 + m] = zp[m]; }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) d1[u][m] = dpsi_z<T>(zz, m);
             }
-            st4(pp, ps);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u && !two) break;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int z = zq + m;
+                    if (z >= zlo && z < zhi) ps[u][m] = (T)bz[m] * ps[u][m] + (T)aa[m] * d1[u][m] * h1;
+                }
+                st4(pp + (u ? ks * pt : 0), ps[u]);
+            }
         }
     }
 }
@@ -386,8 +417,14 @@ struct ResPriv {
 };
 template <typename T>
 struct ResPriv<T, 0> {
-    T cf[1][4];                 // coef of the first column, where it is read from global memory
+    T cf[1][4];                 // coef of the first column, read at every step: tensor memory has the others'
 };
+// Tensor-memory address of coef of a thread's column col >= 1, behind the private values.
+template <typename T>
+__device__ __forceinline__ uint32_t res_coef_at(const ResShape &h, uint32_t tm, int col)
+{
+    return tm + (uint32_t)((h.CW * h.nslot + col - 1) * TmQuad<T>::WORDS);
+}
 
 // The leapfrog of one quad (SRC/stencilDFM.c:17-29): W its 9-column window, zz its z line.
 template <typename T>
@@ -403,8 +440,8 @@ __device__ __forceinline__ void leap_quad(const T (&W)[9][4], const T (&zm)[4], 
 
 // The leapfrog of a thread's columns.  A 9-column register window along x, the column loop unrolled
 // so that the window turns without moves: 3 new 16-byte shared loads a quad and two of tensor memory,
-// a column ahead (previous field, coef).  Where tensor memory has no room for coef it comes from the
-// second-level cache two columns ahead.  The new values go to tensor memory, over the previous field
+// a column ahead (previous field, coef; from the second-level cache, coef made a column take 420 ns
+// instead of 330).  The new values go to tensor memory, over the previous field
 // they consume (res_store swaps them into the tile): held in registers until the block has read the
 // old tile they would spill, and a spill misses the little first-level cache that the tiles leave.
 template <typename T, int NC>
@@ -437,20 +474,10 @@ __device__ __forceinline__ void res_leap(const ResJob<T> &J, const ResCta &c, co
                 for (int j = 0; j < 4; ++j) W[m][j] = W[m + 1][j];
         }
     } else {
-        const size_t P = (size_t)J.g.pitch;
-        const T *cp = J.coef + (size_t)(c.xa + th.xk) * P + c.za + 4 * th.q;
         const uint32_t cstep = (uint32_t)(h.nslot * QW);
-        const bool ctm = h.cslot >= 0;
-        uint32_t ta = tm + (uint32_t)(f * QW), tac = tm + (uint32_t)(max(h.cslot, 0) * QW);
+        uint32_t ta = tm + (uint32_t)(f * QW), tac = res_coef_at<T>(h, tm, 1);
         TmQuad<T> tp, tc;
-        T cfn[2][4];
         tp.load(ta);
-        tc.load(tac);
-        if (!ctm) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cfn[0][j] = me.cf[0][j];
-            ldg4(cp + (cw > 1 ? P : 0), cfn[1]);
-        }
 #pragma unroll
         for (int m = 0; m < 8; ++m) ld4(row + m * sp, W[m]);
 #pragma unroll
@@ -460,19 +487,17 @@ __device__ __forceinline__ void res_leap(const ResJob<T> &J, const ResCta &c, co
             ld4(row + 4 * sp - 4, zm);
             ld4(row + 4 * sp + 4, zp);
             tp.wait(prv);
-            tc.wait(cf);
+            if (u > 0) tc.wait(cf);
+            else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cf[j] = me.cf[0][j];
+            }
             const uint32_t to = ta;
             ta += cstep;
             if (u + 1 < cw) {
                 tp.load(ta);
-                tac += cstep;
                 tc.load(tac);
-            }
-            if (!ctm) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) cf[j] = cfn[u & 1][j];
-                if (u + 2 < cw) ldg4(cp + 2 * P, cfn[u & 1]);
-                cp += P;
+                tac += QW;
             }
             leap_quad<T>(W, zm, zp, cf, prv, v);
             TmQuad<T>::store(to, v);
@@ -671,33 +696,43 @@ __device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
-// With the values in tensor memory each strip is a pass of its own, in the same order.  Left (side 0)
-// and right (1) strips: the columns of the thread that lie in them.
+// With the values in tensor memory each strip is a pass of its own, in the same order, two columns at
+// a time so that one's loads cover the other's arithmetic, and without branches: lanes outside the
+// strip work on the strip's nearest quad and keep their values.
+// Left (side 0) and right (1) strips: the columns of the thread that lie in them.
 template <typename T>
 __device__ __forceinline__ void res_strip_x(const ResJob<T> &J, const ResCta &c, const ResShape &h, const ResThread &th,
-                                            int side, const T *su, const T *sm, const float *px, uint32_t tm)
+                                            int side, const T *su, const T *sm, const float *px, uint32_t tm,
+                                            const T (&cf0)[4])
 {
-    constexpr int QW = TmQuad<T>::WORDS;
-    const uint32_t cstep = (uint32_t)(h.nslot * QW), ox = (uint32_t)(h.xslot * QW), oc = (uint32_t)(h.cslot * QW);
-    const int sp = h.SP, ph = h.PH, cw = h.CW, zl = J.g.dimz - 4 - c.za - 4 * th.q;   // cells before the frame
+    constexpr int QW = TmQuad<T>::WORDS, U = 2;
+    const uint32_t cstep = (uint32_t)(h.nslot * QW), ox = (uint32_t)(h.xslot * QW);
+    const int sp = h.SP, ph = h.PH, zl = J.g.dimz - 4 - c.za - 4 * th.q;              // cells before the frame
     const T h1 = J.h1, h2 = J.h2, h3 = J.h3;
     const int beg = side == 0 ? 0 : h.cr0 - c.xa, end = side == 0 ? h.nl : h.W;       // columns of the block
-    const T *up = su + (th.xk + kResPad) * sp + kResPad + 4 * th.q;
-    const T *ps = sm + (side == 0 ? h.offl : h.offr) + (th.xk - beg + 4) * ph + 4 * th.q;
-    const float2 *pr = reinterpret_cast<const float2 *>(px) + th.xk + 4;
+    // the warp's columns of the strip (a lane's chunk may start a chunk further on)
+    const int lo = __reduce_min_sync(0xffffffffu, max(0, beg - th.xk));
+    const int hi = __reduce_max_sync(0xffffffffu, min(h.CW, end - th.xk));
+    const T *ub = su + kResPad * sp + kResPad + 4 * th.q;
+    const T *pb = sm + (side == 0 ? h.offl : h.offr) + 4 * th.q;
+    const float2 *pr = reinterpret_cast<const float2 *>(px) + 4;
     const T bk[4] = {(T)RTM_B4, (T)RTM_B3, (T)RTM_B2, (T)RTM_B1};
     const T ak[4] = {(T)RTM_AC4, (T)RTM_AC3, (T)RTM_AC2, (T)RTM_AC1};
 #pragma unroll 1
-    for (int xc = th.xk; xc < th.xk + cw; ++xc, up += sp, ps += ph, ++pr, tm += cstep) {
-        const bool in = xc >= beg && xc < end;
-        if (!__any_sync(0xffffffffu, in)) continue;
-        TmQuad<T> tv, tc, tx;
-        T cf[4], v[4], xx[4], acc[4] = {(T)0, (T)0, (T)0, (T)0}, d2[4] = {(T)0, (T)0, (T)0, (T)0};
-        tv.load(tm);
-        tc.load(tm + oc);
-        tx.load(tm + ox);
-        float2 ab = make_float2(0.0f, 0.0f);
-        if (in) {
+    for (int col = lo; col < hi; col += U) {
+        TmQuad<T> tv[U], tc[U], tx[U];
+        T acc[U][4], d2[U][4];
+        float2 ab[U];
+        bool in[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int cc = min(col + u, hi - 1);
+            tv[u].load(tm + cc * cstep);
+            tc[u].load(res_coef_at<T>(h, tm, max(cc, 1)));
+            tx[u].load(tm + cc * cstep + ox);
+            const int xc = th.xk + cc, xs = min(max(xc, beg), end - 1);
+            in[u] = xc == xs && col + u < hi;
+            const T *up = ub + xs * sp, *ps = pb + (xs - beg + 4) * ph;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 T mk[4], pk[4], um[4], uq[4];
@@ -708,63 +743,80 @@ __device__ __forceinline__ void res_strip_x(const ResJob<T> &J, const ResCta &c,
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const T term = bk[k] * (pk[j] - mk[j]);
-                    acc[j] = k == 0 ? term : acc[j] + term;
+                    acc[u][j] = k == 0 ? term : acc[u][j] + term;
                     const T dterm = ak[k] * (uq[j] + um[j]);
-                    d2[j] = k == 0 ? dterm : d2[j] + dterm;
+                    d2[u][j] = k == 0 ? dterm : d2[u][j] + dterm;
                 }
             }
             T uc[4];
             ld4(up, uc);
-            ab = *pr;
+            ab[u] = pr[xs];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) d2[j] = d2[j] + (T)RTM_AC0 * uc[j];
+            for (int j = 0; j < 4; ++j) d2[u][j] = d2[u][j] + (T)RTM_AC0 * uc[j];
         }
-        __syncwarp();
-        tv.wait(v);
-        tc.wait(cf);
-        tx.wait(xx);
-        if (in) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < zl) {
-                    const T dp = acc[j] * h1;
-                    const T xn = (T)ab.y * xx[j] + (T)ab.x * (d2[j] * h3 + dp);
-                    xx[j] = xn;
-                    v[j] = v[j] + mul_rn(cf[j] * h2, dp + xn);
-                }
+        for (int u = 0; u < U; ++u) {
+            T v[4], cf[4], xx[4];
+            tv[u].wait(v);
+            tc[u].wait(cf);
+            tx[u].wait(xx);
+            if (col + u == 0) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cf[j] = cf0[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const T dp = acc[u][j] * h1;
+                const T xn = (T)ab[u].y * xx[j] + (T)ab[u].x * (d2[u][j] * h3 + dp);
+                const T vn = v[j] + mul_rn(cf[j] * h2, dp + xn);
+                const bool ok = in[u] && j < zl;
+                xx[j] = ok ? xn : xx[j];
+                v[j] = ok ? vn : v[j];
+            }
+            if (u == 0 || col + u < hi) {
+                TmQuad<T>::store(tm + (col + u) * cstep, v);
+                TmQuad<T>::store(tm + (col + u) * cstep + ox, xx);
+            }
         }
-        __syncwarp();
-        TmQuad<T>::store(tm, v);
-        TmQuad<T>::store(tm + ox, xx);
     }
 }
 // Top (side 2) and bottom (3) strips: all of the thread's columns, if its rows lie in them.
 template <typename T>
 __device__ __forceinline__ void res_strip_z(const ResJob<T> &J, const ResCta &c, const ResShape &h, const ResThread &th,
-                                            int side, const T *su, const T *sm, const float *pz, uint32_t tm)
+                                            int side, const T *su, const T *sm, const float *pz, uint32_t tm,
+                                            const T (&cf0)[4])
 {
-    constexpr int QW = TmQuad<T>::WORDS;
+    constexpr int QW = TmQuad<T>::WORDS, U = sizeof(T) == 4 ? 2 : 1;
     const Geom &g = J.g;
-    const uint32_t cstep = (uint32_t)(h.nslot * QW), oz = (uint32_t)(h.zslot * QW), oc = (uint32_t)(h.cslot * QW);
-    const int sp = h.SP, cw = h.CW, zq = c.za + 4 * th.q, pt = side == 2 ? h.PT : h.PB;
+    const uint32_t cstep = (uint32_t)(h.nslot * QW), oz = (uint32_t)(h.zslot * QW);
+    const int sp = h.SP, cw = h.CW, pt = side == 2 ? h.PT : h.PB;
     const T h1 = J.h1, h2 = J.h2, h3 = J.h3;
     const int zlo = side == 2 ? 4 : g.dimz - g.thd + 4, zhi = side == 2 ? g.thu - 4 : g.dimz - 4;
-    const bool in = zq < zhi && zq + 4 > zlo;
-    if (!__any_sync(0xffffffffu, in)) return;
-    const T *up = su + (th.xk + kResPad) * sp + kResPad + 4 * th.q;
-    const T *ps = sm + (side == 2 ? h.offt : h.offb) + th.xk * pt + (zq - ((side == 2 ? h.qt0 : h.qb0) - 4));
+    const int zq = c.za + 4 * th.q, first = side == 2 ? h.qt0 : h.qb0, count = side == 2 ? h.ht : h.hb;
+    const int zs = min(max(zq, first), first + count - 4);                            // the strip's nearest quad
+    if (!__any_sync(0xffffffffu, zs == zq)) return;
+    const T *ub = su + kResPad * sp + kResPad + (zs - c.za);
+    const T *pb = sm + (side == 2 ? h.offt : h.offb) + (zs - first + 4);
     float aa[4], bz[4];
-    ld4(pz + 2 * (4 * th.q + kResPad), aa);
-    ld4(pz + 2 * (4 * th.q + kResPad) + 4, bz);
-    const int last = h.W - 1 - th.xk;                     // the spare column repeats the block's last one
+    ld4(pz + 2 * (zs - c.za + kResPad), aa);
+    ld4(pz + 2 * (zs - c.za + kResPad) + 4, bz);
+    bool up_j[4], frame[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        up_j[j] = zs == zq && zq + j >= zlo && zq + j < zhi;
+        frame[j] = zq + j >= g.dimz - 4;
+    }
 #pragma unroll 1
-    for (int col = 0; col < cw; ++col, tm += cstep) {
-        TmQuad<T> tv, tc, tz;
-        T cf[4], v[4], xz[4], dp[4], d2[4];
-        tv.load(tm);
-        tc.load(tm + oc);
-        tz.load(tm + oz);
-        if (in) {
+    for (int col = 0; col < cw; col += U) {
+        TmQuad<T> tv[U], tc[U], tz[U];
+        T dp[U][4], d2[U][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int cc = min(col + u, cw - 1), xc = min(th.xk + cc, h.W - 1);       // (the spare column)
+            tv[u].load(tm + cc * cstep);
+            tc[u].load(res_coef_at<T>(h, tm, max(cc, 1)));
+            tz[u].load(tm + cc * cstep + oz);
+            const T *up = ub + xc * sp, *ps = pb + xc * pt;
             T q[12], zz[12], a0[4], a1[4], a2[4];
             ld4(ps - 4, a0);
             ld4(ps, a1);
@@ -778,31 +830,33 @@ __device__ __forceinline__ void res_strip_z(const ResJob<T> &J, const ResCta &c,
             for (int j = 0; j < 4; ++j) { zz[j] = a0[j]; zz[4 + j] = a1[j]; zz[8 + j] = a2[j]; }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                dp[j] = dpsi_z<T>(q, j);
-                d2[j] = d2z_q<T>(zz, j);
+                dp[u][j] = dpsi_z<T>(q, j);
+                d2[u][j] = d2z_q<T>(zz, j);
             }
         }
-        __syncwarp();
-        tv.wait(v);
-        tc.wait(cf);
-        tz.wait(xz);
-        if (in) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            T v[4], cf[4], xz[4];
+            tv[u].wait(v);
+            tc[u].wait(cf);
+            tz[u].wait(xz);
+            if (col + u == 0) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cf[j] = cf0[j];
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int z = zq + j;
-                if (z >= zlo && z < zhi) {
-                    const T d1 = dp[j] * h1;
-                    const T xn = (T)bz[j] * xz[j] + (T)aa[j] * (d2[j] * h3 + d1);
-                    xz[j] = xn;
-                    v[j] = v[j] + mul_rn(cf[j] * h2, d1 + xn);
-                }
-                if (z >= g.dimz - 4) v[j] = (T)0;         // the grid's frame stays zero
+                const T d1 = dp[u][j] * h1;
+                const T xn = (T)bz[j] * xz[j] + (T)aa[j] * (d2[u][j] * h3 + d1);
+                const T vn = v[j] + mul_rn(cf[j] * h2, d1 + xn);
+                xz[j] = up_j[j] ? xn : xz[j];
+                v[j] = frame[j] ? (T)0 : up_j[j] ? vn : v[j];                        // the grid's frame stays zero
+            }
+            if (u == 0 || col + u < cw) {
+                TmQuad<T>::store(tm + (col + u) * cstep, v);
+                TmQuad<T>::store(tm + (col + u) * cstep + oz, xz);
             }
         }
-        __syncwarp();
-        TmQuad<T>::store(tm, v);
-        TmQuad<T>::store(tm + oz, xz);
-        if (col < last) { up += sp; ps += pt; }
     }
 }
 // ... of all of a thread's columns.
@@ -825,11 +879,11 @@ __device__ __forceinline__ void res_strips(const ResJob<T> &J, const ResCta &c, 
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {                     // left, top; right, bottom
             if (k == 0 ? h.nl : h.nr) {
-                res_strip_x<T>(J, c, h, th, k, su, sm, px, tm);
+                res_strip_x<T>(J, c, h, th, k, su, sm, px, tm, me.cf[0]);
                 tm_wait_st();
             }
             if (k == 0 ? h.ht : h.hb) {
-                res_strip_z<T>(J, c, h, th, 2 + k, su, sm, pz, tm);
+                res_strip_z<T>(J, c, h, th, 2 + k, su, sm, pz, tm, me.cf[0]);
                 tm_wait_st();
             }
         }
@@ -1076,9 +1130,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if constexpr (NC == 0) {
             TmQuad<T>::store(tm + col * cstep, q);
             if (two) TmQuad<T>::store(tm + col * cstep + QW, p2);
-            if (h.cslot >= 0) {
+            if (col > 0) {
                 ldg4(J.coef + (size_t)x * P + zq, q);
-                TmQuad<T>::store(tm + col * cstep + h.cslot * QW, q);
+                TmQuad<T>::store(res_coef_at<T>(h, tm, col), q);
             }
         } else {
 #pragma unroll
@@ -1175,8 +1229,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
             cp_async_commit();
         }
-        if constexpr (NC == 0)
-            if (h.cslot < 0) ldg4(J.coef + (size_t)(c.xa + th.xk) * P + zq, me.cf[0]);
+        if constexpr (NC == 0) ldg4(J.coef + (size_t)(c.xa + th.xk) * P + zq, me.cf[0]);
         bool ok = true;
         if (t > t0) ok = res_recv<T>(c, tid, in, t >= 3 ? nin : nin0, tag, xch, sm, status);
         if constexpr (NC == 0) tm_wait_st();
@@ -1242,7 +1295,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
             __syncthreads();
         }
-        if (t + 1 < t1) res_send<T>(c, tid, out, recon ? nout : nout0, tag + 1, xch, sm);
+        if (t + 1 < t1) res_send<T, (NC == 0 && sizeof(T) == 4 ? 2 : 1)>(c, tid, out, recon ? nout : nout0, tag + 1, xch, sm);
         // ---- storage of the forward field, image of the backward ones
         if (!back && ring && t + 1 < g.nt) {            // slot k holds the ring of u_k
             T *slot = store + (size_t)(t + 1) * J.slot_elems;
@@ -1268,9 +1321,13 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 T q[4];
                 ld4(own + col * h.SP, q);
                 if (!back) {
+                    if (zfull) {
+                        st4(slot + o, q);
+                        continue;
+                    }
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        if (zfull || in_interior(g, x, zq + j)) slot[o + j] = q[j];
+                        if (in_interior(g, x, zq + j)) slot[o + j] = q[j];
                     continue;
                 }
                 T s[4];
