@@ -225,19 +225,28 @@ __device__ __forceinline__ unsigned halo_item(const ResShape &h, const ResHalo &
     const int at = (f ? h.field : 0) + (x + kResPad) * h.SP + kResPad + z;
     return (unsigned)(at >> 2) | (unsigned)side << 15 | f << 17 | (unsigned)quad << 18;
 }
-// The item's words at parity par; off / cap: the sides' mailboxes.
-template <typename T>
-__device__ __forceinline__ size_t halo_word(const unsigned (&off)[4], const int (&cap)[4], unsigned item, int par)
+// Mailboxes of the block, by parity, field and side: the address of each one's first quad.
+struct ResBox {
+    unsigned long long *at[16];
+};
+__device__ __forceinline__ unsigned long long *res_box(const unsigned (&off)[4], const int (&cap)[4], int i, unsigned long long *xch,
+                                                       int words)
 {
-    const unsigned side = (item >> 15) & 3u, f = (item >> 17) & 1u;
-    return (size_t)(off[side] + (2 * f + par) * (unsigned)cap[side] + (item >> 18)) * kXWords<T>;
+    const int side = i & 3, f = (i >> 2) & 1, par = i >> 3;
+    return xch + (size_t)(off[side] + (unsigned)((2 * f + par) * cap[side])) * words;
+}
+// The item's words at parity par.
+template <typename T>
+__device__ __forceinline__ unsigned long long *halo_word(const ResBox &b, unsigned item, int par)
+{
+    return b.at[par * 8 + ((item >> 15) & 7u)] + (item >> 18) * kXWords<T>;
 }
 
 // Receives the first n items of the halo (this thread's: in[k] = item tid + k kResThreads); false
 // when a wait ran out.  Two items a round: their loads are in flight together.
 template <typename T>
-__device__ __forceinline__ bool res_recv(const ResCta &c, int tid, const unsigned (&in)[kResItems], int n, unsigned tag,
-                                         const unsigned long long *xch, T *tile, const unsigned *status)
+__device__ __forceinline__ bool res_recv(const ResBox &b, int tid, const unsigned (&in)[kResItems], int n, unsigned tag,
+                                         T *tile, const unsigned *status)
 {
     const int par = (int)(tag & 1u);
     bool ok = true;
@@ -251,7 +260,7 @@ __device__ __forceinline__ bool res_recv(const ResCta &c, int tid, const unsigne
         for (int k = 0; k < 2; ++k) {
             have[k] = tid + (r + k) * kResThreads < n;
             if (have[k]) {
-                p[k] = xch + halo_word<T>(c.in_off, c.in_cap, in[r + k], par);
+                p[k] = halo_word<T>(b, in[r + k], par);
                 x[k].load(p[k]);
             }
         }
@@ -269,8 +278,8 @@ __device__ __forceinline__ bool res_recv(const ResCta &c, int tid, const unsigne
 
 // Publishes the first n items that the neighbours need, R a round: their loads are in flight together.
 template <typename T, int R>
-__device__ __forceinline__ void res_send(const ResCta &c, int tid, const unsigned (&out)[kResItems], int n, unsigned tag,
-                                         unsigned long long *xch, const T *tile)
+__device__ __forceinline__ void res_send(const ResBox &b, int tid, const unsigned (&out)[kResItems], int n, unsigned tag,
+                                         const T *tile)
 {
     const int par = (int)(tag & 1u);
 #pragma unroll
@@ -283,7 +292,7 @@ __device__ __forceinline__ void res_send(const ResCta &c, int tid, const unsigne
 #pragma unroll
         for (int k = 0; k < R; ++k)
             if (tid + (r + k) * kResThreads < n)
-                x_put<T>(xch + halo_word<T>(c.out_off, c.out_cap, out[r + k], par), q[k], tag);
+                x_put<T>(halo_word<T>(b, out[r + k], par), q[k], tag);
     }
 }
 
@@ -511,77 +520,81 @@ __device__ __forceinline__ void res_leap(const ResJob<T> &J, const ResCta &c, co
     }
 }
 
-// What stays the same for a thread of a strip block at every step, with NC > 0: its psi quads (xn of
-// the left or right strip, zn of the top or bottom one, at a fixed stride) and where the psi of its own
-// quads lies.  Worked out at every step, the index arithmetic and its chain of shared loads took a
+// What stays the same for a thread of a strip block at every step, with NC > 0: its psi quads (a count
+// in the left or right strip and one in the top or bottom one, at a fixed stride of columns) and where
+// the psi of its own quads lies.  Worked out at every step, the index arithmetic and its chain of shared loads took a
 // third of a small grid's step.  (A block that holds both strips of an axis runs with NC = 0.)
+// Packed: they live in registers over all steps, and a word spilt costs a way to the second-level
+// cache at every one (offsets are below 65536: 224 KB hold 57344 values).
 struct ResFix {
-    int xp, xu, xn, xdp, xdu, xr, xdr, xl;    // psi, u (first of the 9 rows), count, strides; profile; cells before the frame
-    int zp, zu, zn, zdp, zdu, zr, zlo, zhi;   // ..., profile; cells [zlo, zhi) of the quad are updated
-    int sx, sz;                               // psi of the thread's first quad in the x / z strip
-    int xm;                                   // columns of the thread in the x strip (bit u)
-    int slo, shi, sl;                         // cells [slo, shi) of its quads lie in the z strip, sl before the frame
-    bool xfirst;                              // the x correction comes before the z one
+    unsigned x, z;              // psi (low half), u (high half) of the first x / z quad; u at the first of its rows
+    unsigned xw, zw;            // profile's column or quad (10 bits), stride in columns (10), count (9), x: cells before the frame (3)
+    unsigned s;                 // psi of the thread's own first quad in the x (low) and z strip
+    unsigned bits;              // zlo 3, zhi 3: cells of the z quad; slo 3, shi 3: ... of its own quads in the z strip;
+                                // sl 3: their cells before the frame; xm 2: its columns in the x strip; xfirst 1
+    __device__ __forceinline__ int get(int at, int n) const { return (int)((bits >> at) & ((1u << n) - 1u)); }
+    __device__ __forceinline__ int zlo() const { return get(0, 3); }
+    __device__ __forceinline__ int zhi() const { return get(3, 3); }
+    __device__ __forceinline__ int slo() const { return get(6, 3); }
+    __device__ __forceinline__ int shi() const { return get(9, 3); }
+    __device__ __forceinline__ int sl() const { return get(12, 3); }
+    __device__ __forceinline__ bool in_x(int u) const { return get(15 + u, 1); }
+    __device__ __forceinline__ bool xfirst() const { return get(17, 1); }
 };
 __device__ __forceinline__ void res_fix_init(const Geom &g, const ResCta &c, const ResShape &h, const ResPsi &w,
                                              const ResThread &th, int tid, ResFix &f)
 {
-    f.xn = f.zn = f.xm = 0;
-    f.sx = f.sz = -1;
-    f.xp = f.xu = f.xdp = f.xdu = f.xr = f.xdr = f.xl = f.zp = f.zu = f.zdp = f.zdu = f.zr = f.zlo = f.zhi = 0;
-    f.slo = f.shi = 0;
-    f.xfirst = true;
+    auto cells = [](int n) { return (unsigned)min(max(n, 0), 4); };
+    f.x = f.z = f.xw = f.zw = f.s = 0u;
     const int zq = c.za + 4 * th.q;
-    f.sl = g.dimz - 4 - zq;
+    f.bits = cells(g.dimz - 4 - zq) << 12 | 1u << 17;
+    int first = 0;              // threads with quads of the x strip, in whole warps
     if (h.nl || h.nr) {
         const int side = h.nl ? 0 : 1, rows = w.rows[side], ks = kResThreads / rows, k = tid / rows, q = tid - k * rows;
         const int x = w.lo[side] + k;
         if (k < ks && x < w.hi[side]) {
-            f.xp = (side ? h.offr + (x - h.cr0 + 4) * h.PH : h.offl + (x - h.cl0 + 4) * h.PH) + 4 * q;
-            f.xu = (x - 4 - c.xa + kResPad) * h.SP + kResPad + 4 * q;
-            f.xr = x - c.xa + 4;
-            f.xn = (w.hi[side] - x + ks - 1) / ks;
-            f.xdp = ks * h.PH;
-            f.xdu = ks * h.SP;
-            f.xdr = ks;
-            f.xl = g.dimz - 4 - (c.za + 4 * q);
+            f.x = (unsigned)((side ? h.offr + (x - h.cr0 + 4) * h.PH : h.offl + (x - h.cl0 + 4) * h.PH) + 4 * q) |
+                  (unsigned)((x - 4 - c.xa + kResPad) * h.SP + kResPad + 4 * q) << 16;
+            f.xw = (unsigned)(x - c.xa + 4) | (unsigned)ks << 10 | (unsigned)((w.hi[side] - x + ks - 1) / ks) << 20 |
+                   cells(g.dimz - 4 - (c.za + 4 * q)) << 29;
         }
         const int x0 = c.xa + th.xk;
         for (int u = 0; u < 2; ++u)
-            if (side == 0 ? x0 + u < g.thl - 4 : x0 + u >= g.dimx - g.thr + 4) f.xm |= 1 << u;
-        f.sx = (side ? h.offr + (x0 - h.cr0 + 4) * h.PH : h.offl + (x0 - h.cl0 + 4) * h.PH) + 4 * th.q;
+            if (side == 0 ? x0 + u < g.thl - 4 : x0 + u >= g.dimx - g.thr + 4) f.bits |= 1u << (15 + u);
+        if (f.bits & (3u << 15)) f.s = (unsigned)((side ? h.offr + (x0 - h.cr0 + 4) * h.PH : h.offl + (x0 - h.cl0 + 4) * h.PH) + 4 * th.q);
+        first = min(kResThreads, ((w.hi[side] - w.lo[side]) * rows + 31) & ~31);
     }
     if (h.ht || h.hb) {
-        const int side = h.ht ? 2 : 3, rows = w.rows[side], ks = kResThreads / rows, k = tid / rows, q = tid - k * rows;
+        // the threads after those of the x strip come first: a corner's two kinds run side by side
+        const int turn = (tid - first) & (kResThreads - 1);
+        const int side = h.ht ? 2 : 3, rows = w.rows[side], ks = kResThreads / rows, k = turn / rows, q = turn - k * rows;
         const int zp = w.lo[side] + 4 * q, pt = side == 2 ? h.PT : h.PB, off = side == 2 ? h.offt : h.offb;
         const int q0 = (side == 2 ? h.qt0 : h.qb0) - 4;
         const int zlo = side == 2 ? 4 : g.dimz - g.thd + 4, zhi = side == 2 ? g.thu - 4 : g.dimz - 4;
         if (k < ks && k < h.W) {
-            f.zp = off + k * pt + (zp - q0);
-            f.zu = (k + kResPad) * h.SP + kResPad + (zp - c.za);
-            f.zr = 2 * (zp - c.za + kResPad);
-            f.zn = (h.W - k + ks - 1) / ks;
-            f.zdp = ks * pt;
-            f.zdu = ks * h.SP;
-            f.zlo = zlo - zp;
-            f.zhi = zhi - zp;
+            f.z = (unsigned)(off + k * pt + (zp - q0)) | (unsigned)((k + kResPad) * h.SP + kResPad + (zp - c.za)) << 16;
+            f.zw = (unsigned)((zp - c.za + kResPad) >> 2) | (unsigned)ks << 10 | (unsigned)((h.W - k + ks - 1) / ks) << 20;
+            f.bits |= cells(zlo - zp) | cells(zhi - zp) << 3;
         }
-        f.slo = zlo - zq;
-        f.shi = zhi - zq;
-        if (f.slo < 4 && f.shi > 0) f.sz = off + th.xk * pt + (zq - q0);
-        else f.slo = f.shi = 0;
-        f.xfirst = h.nl || side == 3;
+        if (zlo - zq < 4 && zhi - zq > 0) {
+            f.s |= (unsigned)(off + th.xk * pt + (zq - q0)) << 16;
+            f.bits |= cells(zlo - zq) << 6 | cells(zhi - zq) << 9;
+        }
+        if (!h.nl && side != 3) f.bits &= ~(1u << 17);
     }
 }
 template <typename T>
-__device__ __forceinline__ void res_psi_fix(const ResFix &f, T h1, int sp, const T *su, T *sm, const float *px, const float *pz)
+__device__ __forceinline__ void res_psi_fix(const ResFix &f, const ResShape &h, T h1, const T *su, T *sm, const float *px,
+                                            const float *pz)
 {
-    {
-        T *pp = sm + f.xp;
-        const T *up = su + f.xu;
-        const float2 *pr = reinterpret_cast<const float2 *>(px) + f.xr;
+    const int sp = h.SP;
+    if (f.xw) {
+        const int ks = (int)((f.xw >> 10) & 1023u), ph = h.PH, xl = (int)(f.xw >> 29);
+        T *pp = sm + (f.x & 0xffffu);
+        const T *up = su + (f.x >> 16);
+        const float2 *pr = reinterpret_cast<const float2 *>(px) + (f.xw & 1023u);
 #pragma unroll 1
-        for (int i = 0; i < f.xn; ++i, pp += f.xdp, up += f.xdu, pr += f.xdr) {
+        for (int i = (int)((f.xw >> 20) & 511u); i > 0; --i, pp += ks * ph, up += ks * sp, pr += ks) {
             T ps[4], W[9][4];
             const float2 ab = *pr;
             ld4(pp, ps);
@@ -590,18 +603,19 @@ __device__ __forceinline__ void res_psi_fix(const ResFix &f, T h1, int sp, const
                 if (m != 4) ld4(up + m * sp, W[m]);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (j < f.xl) ps[j] = (T)ab.y * ps[j] + (T)ab.x * d1x_w<T>(W, j) * h1;
+                if (j < xl) ps[j] = (T)ab.y * ps[j] + (T)ab.x * d1x_w<T>(W, j) * h1;
             st4(pp, ps);
         }
     }
-    if (f.zn > 0) {
-        T *pp = sm + f.zp;
-        const T *up = su + f.zu;
+    if (f.zw) {
+        const int ks = (int)((f.zw >> 10) & 1023u), pt = h.ht ? h.PT : h.PB;
+        T *pp = sm + (f.z & 0xffffu);
+        const T *up = su + (f.z >> 16);
         float aa[4], bz[4];
-        ld4(pz + f.zr, aa);
-        ld4(pz + f.zr + 4, bz);
+        ld4(pz + 8 * (f.zw & 1023u), aa);
+        ld4(pz + 8 * (f.zw & 1023u) + 4, bz);
 #pragma unroll 1
-        for (int i = 0; i < f.zn; ++i, pp += f.zdp, up += f.zdu) {
+        for (int i = (int)(f.zw >> 20); i > 0; --i, pp += ks * pt, up += ks * sp) {
             T ps[4], zz[12], zm[4], c4[4], zp[4];
             ld4(pp, ps);
             ld4(up - 4, zm);
@@ -611,7 +625,7 @@ __device__ __forceinline__ void res_psi_fix(const ResFix &f, T h1, int sp, const
             for (int m = 0; m < 4; ++m) { zz[m] = zm[m]; zz[4 + m] = c4[m]; zz[8 + m] = zp[m]; }
 #pragma unroll
             for (int m = 0; m < 4; ++m)
-                if (m >= f.zlo && m < f.zhi) ps[m] = (T)bz[m] * ps[m] + (T)aa[m] * dpsi_z<T>(zz, m) * h1;
+                if (m >= f.zlo() && m < f.zhi()) ps[m] = (T)bz[m] * ps[m] + (T)aa[m] * dpsi_z<T>(zz, m) * h1;
             st4(pp, ps);
         }
     }
@@ -627,7 +641,7 @@ __device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h
                                                T (&xx)[4], T (&xz)[4], T (&v)[4])
 {
     T dX[4] = {(T)0, (T)0, (T)0, (T)0}, dZ[4] = {(T)0, (T)0, (T)0, (T)0}, uc[4];
-    const bool inX = (f.xm >> u) & 1, inZ = f.sz >= 0;
+    const bool inX = f.in_x(u), inZ = f.slo() < f.shi();
     ld4(up, uc);
     if (inX) {
         const T ab = (T)pr.x, bb = (T)pr.y;
@@ -652,7 +666,7 @@ __device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             d2[j] = d2[j] + (T)RTM_AC0 * uc[j];
-            if (j < f.sl) {
+            if (j < f.sl()) {
                 const T dp = acc[j] * h1;
                 const T xn = bb * xx[j] + ab * (d2[j] * h3 + dp);
                 xx[j] = xn;
@@ -676,7 +690,7 @@ __device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h
         for (int j = 0; j < 4; ++j) { zz[j] = a0[j]; zz[4 + j] = uc[j]; zz[8 + j] = a2[j]; }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (j >= f.slo && j < f.shi) {
+            if (j >= f.slo() && j < f.shi()) {
                 const T dp = dpsi_z<T>(q, j) * h1;
                 const T xn = (T)bz[j] * xz[j] + (T)aa[j] * (d2z_q<T>(zz, j) * h3 + dp);
                 xz[j] = xn;
@@ -685,10 +699,10 @@ __device__ __forceinline__ void res_strip_quad(const ResFix &f, int u, T h1, T h
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (inX && f.xfirst) v[j] = v[j] + dX[j];
+        if (inX && f.xfirst()) v[j] = v[j] + dX[j];
         if (inZ) v[j] = v[j] + dZ[j];
-        if (inX && !f.xfirst) v[j] = v[j] + dX[j];
-        if (j >= f.sl) v[j] = (T)0;                      // the grid's frame stays zero
+        if (inX && !f.xfirst()) v[j] = v[j] + dX[j];
+        if (j >= f.sl()) v[j] = (T)0;                      // the grid's frame stays zero
     }
 }
 
@@ -873,7 +887,7 @@ __device__ __forceinline__ void res_strips(const ResJob<T> &J, const ResCta &c, 
 #pragma unroll
         for (int u = 0; u < NC; ++u)
             if (u == 0 || u < th.len)
-                res_strip_quad<T>(f, u, h1, h2, h3, sp, ph, up + u * sp, sm + f.sx + u * ph, sm + f.sz + u * pt, pr[u],
+                res_strip_quad<T>(f, u, h1, h2, h3, sp, ph, up + u * sp, sm + (f.s & 0xffffu) + u * ph, sm + (f.s >> 16) + u * pt, pr[u],
                                   pz + 2 * (4 * th.q + kResPad), me.cf[u], me.xx[u], me.xz[u], me.v[u]);
     } else {
 #pragma unroll 1
@@ -1175,6 +1189,11 @@ __global__ void __launch_bounds__(kResThreads, 1)
     __syncthreads();
     const int nring = ring ? ring_items(rb) : 0;
     __shared__ ResHalo hin, hout;
+    __shared__ ResBox box_in, box_out;
+    if (tid < 16) {
+        box_in.at[tid] = res_box(c.in_off, c.in_cap, tid, xch, kXWords<T>);
+        box_out.at[tid] = res_box(c.out_off, c.out_cap, tid, xch, kXWords<T>);
+    }
     if (tid < 4) {
         hin.d[tid] = c.din[tid];
         hout.d[tid] = c.dout[tid];
@@ -1205,15 +1224,17 @@ __global__ void __launch_bounds__(kResThreads, 1)
     bool dead = false;
     for (int t = t0; t < t1; ++t) {
         const unsigned tag = tag0 + (unsigned)(t - t0);     // of the fields this step reads
-        if constexpr (NC == 0) {
-            opaque(tid);
-            opaque(zq);
-            opaque(th.q);
-            opaque(th.xk);
-            opaque(th.len);
+        // (what the compiler worked out of these ahead of the loop it kept in spilt words: 96 x 64
+        // 2.69 -> 2.40 us a step, 400 x 200 2.92 -> 2.76, and NC = 0 the more so)
+        opaque(tid);
+        opaque(zq);
+        opaque(th.q);
+        opaque(th.xk);
+        opaque(th.len);
 #pragma unroll
-            for (int k = 0; k < kResItems; ++k) { opaque(in[k]); opaque(out[k]); }
-        }
+        for (int k = 0; k < kResItems; ++k) { opaque(in[k]); opaque(out[k]); }
+        if constexpr (NC > 0)
+            for (unsigned *w : {&fix.x, &fix.z, &fix.xw, &fix.zw, &fix.s, &fix.bits}) opaque(*w);
         const bool recon = hasS && t >= 2;
         // inputs of the step that do not depend on the neighbours
         float seis = 0.0f;
@@ -1231,7 +1252,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         }
         if constexpr (NC == 0) ldg4(J.coef + (size_t)(c.xa + th.xk) * P + zq, me.cf[0]);
         bool ok = true;
-        if (t > t0) ok = res_recv<T>(c, tid, in, t >= 3 ? nin : nin0, tag, xch, sm, status);
+        if (t > t0) ok = res_recv<T>(box_in, tid, in, t >= 3 ? nin : nin0, tag, sm, status);
         if constexpr (NC == 0) tm_wait_st();
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicOr(status, ST_TMA_TIMEOUT);
@@ -1239,7 +1260,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             break;
         }
         if constexpr (NC > 0) {
-            if (strip) res_psi_fix<T>(fix, J.h1, h.SP, su, sm, px, pz);
+            if (strip) res_psi_fix<T>(fix, h, J.h1, su, sm, px, pz);
         } else {
             if (strip) res_psi<T>(J, c, h, wpsi, tid, su, sm, px, pz);
         }
@@ -1295,7 +1316,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
             __syncthreads();
         }
-        if (t + 1 < t1) res_send<T, (NC == 0 && sizeof(T) == 4 ? 2 : 1)>(c, tid, out, recon ? nout : nout0, tag + 1, xch, sm);
+        if (t + 1 < t1) res_send<T, (NC == 0 && sizeof(T) == 4 ? 2 : 1)>(box_out, tid, out, recon ? nout : nout0, tag + 1, sm);
         // ---- storage of the forward field, image of the backward ones
         if (!back && ring && t + 1 < g.nt) {            // slot k holds the ring of u_k
             T *slot = store + (size_t)(t + 1) * J.slot_elems;
