@@ -131,7 +131,11 @@ inline bool res_partition(const Geom &g, int fields, int es, int sms, ResPart &o
                 cw = std::max(cw, (s.nl && s.nr) || (s.ht && s.hb) ? std::max(3, s.CW) : s.CW);
                 smem = std::max(smem, res_bytes(s, es));
             }
-        if (cw == 2 && es == 4) cost *= 1.2;         // two columns in registers (k_resident's NC) against one
+        // a step with two columns in registers (k_resident's NC), or more in tensor memory, against one:
+        // 400 x 200 2.84 us with one, 3.22 with two; 901 x 301 4.14 with two, 5.57 with more, 600 x 300
+        // 4.22 and 1600 x 100 4.50 with two (1.2 and any factor from 1.3 to 1.6 choose the better there
+        // and on 11 more grids; 2.0 takes 1201 x 403 from 6.04 to 6.38)
+        if (es == 4) cost *= cw == 1 ? 1.0 : cw == 2 ? 1.2 : 1.5;
         return cost < most;
     };
     const double cells = (double)(X1 - X0) * (Z1 - Z0);
