@@ -8,6 +8,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "rtm_internal.h"
@@ -79,6 +80,12 @@ inline double res_cost(const ResShape &s, int fields, int es)
 
 inline size_t res_bytes(const ResShape &s, int es) { return es == 8 ? res_smem<double>(s) : res_smem<float>(s); }
 
+// A step with two columns in registers (k_resident's NC), or more in tensor memory, against one:
+// 400 x 200 2.84 us with one, 3.22 with two; 901 x 301 4.14 with two, 5.57 with more, 600 x 300
+// 4.22 and 1600 x 100 4.50 with two (1.2 and any factor from 1.3 to 1.6 choose the better there
+// and on 11 more grids; 2.0 takes 1201 x 403 from 6.04 to 6.38).
+inline double res_kind(int cw) { return cw == 1 ? 1.0 : cw == 2 ? 1.2 : 1.5; }
+
 // Halo quads of a block in one direction at most: 8 columns or 2 rows of quads of the first field
 // across each side (a neighbour in a strip needs them), 4 and 1 of the second.
 inline int res_halo_most(const ResShape &s) { return 2 * (8 + 4) * s.HQ + 2 * (2 + 1) * s.W; }
@@ -131,11 +138,7 @@ inline bool res_partition(const Geom &g, int fields, int es, int sms, ResPart &o
                 cw = std::max(cw, (s.nl && s.nr) || (s.ht && s.hb) ? std::max(3, s.CW) : s.CW);
                 smem = std::max(smem, res_bytes(s, es));
             }
-        // a step with two columns in registers (k_resident's NC), or more in tensor memory, against one:
-        // 400 x 200 2.84 us with one, 3.22 with two; 901 x 301 4.14 with two, 5.57 with more, 600 x 300
-        // 4.22 and 1600 x 100 4.50 with two (1.2 and any factor from 1.3 to 1.6 choose the better there
-        // and on 11 more grids; 2.0 takes 1201 x 403 from 6.04 to 6.38)
-        if (es == 4) cost *= cw == 1 ? 1.0 : cw == 2 ? 1.2 : 1.5;
+        if (es == 4) cost *= res_kind(cw);
         return cost < most;
     };
     const double cells = (double)(X1 - X0) * (Z1 - Z0);
@@ -143,7 +146,9 @@ inline bool res_partition(const Geom &g, int fields, int es, int sms, ResPart &o
     int px_of_kx = -1;
     for (int pz = 1; pz <= std::min(sms, std::max(1, (Z1 - Z0) / 8)); ++pz) {
         const int px = std::min(sms / pz, std::max(1, (X1 - X0) / 8));
-        if (found && cells / (4.0 * kResThreads * px * pz) * fields * (es == 8 ? 1.0 : 430.0) > out.cost) continue;
+        const double quads = cells / (4.0 * kResThreads * px * pz);       // a thread's, of the mean block
+        const int least = std::max(1, (int)std::ceil(quads - 1e-9));
+        if (found && (es == 8 ? quads * fields : least * fields * 430.0 * res_kind(least)) > out.cost) continue;
         for (int w = 0; w < 7; ++w)
             kinds(res_cuts(Z0, Z1, g.thu - 4, g.dimz - g.thd + 4, weights[w], pz, 4), g.thu - 4, g.dimz - g.thd + 4, g.rz0,
                   g.rz1, kz[w]);
