@@ -31,7 +31,6 @@ sys.path.insert(0, ROOT)
 
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6800.0
-TRAFFIC_SUMMARY = os.path.join(ROOT, "profiles", "k_step_bwd_traffic.txt")
 
 
 def parse():
@@ -53,8 +52,10 @@ def parse():
     ap.add_argument("--batch-members", type=int, default=64,
                     help="batched UQ ensemble: velocity realizations (0: skip)")
     ap.add_argument("--batch-nt", type=int, default=7500)
+    ap.add_argument("--batch-autotune", action="store_true",
+                    help="batched members on the step kernels, at a tuned tile width (default: resident passes)")
     ap.add_argument("--no-batch-autotune", dest="batch_autotune", action="store_false",
-                    help="batched members at the default 32-column tile width")
+                    help="the default")
     ap.add_argument("--plain-sample", type=int, default=6,
                     help="ensemble members also run one at a time through the plain path")
     ap.add_argument("--serve-requests", type=int, default=96,
@@ -180,24 +181,31 @@ def algorithmic_bytes(p):
     return {"k_step_fwd": fwd, "k_step_bwd": bwd, "k_bpsi": 12 * psi, "batched_fwd_step": batched_fwd}
 
 
+def flops_per_step(p):
+    """Operations of one time step: 25 a cell and field for the leapfrog, 50 more a CPML cell, 4 an
+    imaged cell (the reconstructed source field covers the interior and 4 cells around it)."""
+    cells, interior = p.dim_x * p.dim_z, p.nx * p.nz
+    fwd = 25 * cells + 50 * (cells - interior)
+    return fwd, fwd + 25 * (p.nx + 8) * (p.nz + 8) + 4 * interior / p.time_slices
+
+
+def fp32_peak():
+    """Nominal FP32 rate (TFLOP/s): 128 fused multiply-adds a cycle and SM at the highest clock."""
+    import torch
+    try:
+        with open(MEASURED_PEAKS) as f:
+            mhz = float(json.load(f)["sm_max_mhz"])
+    except Exception:
+        mhz = 2070.0
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count * 256 * mhz * 1e-6
+
+
 def hbm_peak():
     try:
         with open(MEASURED_PEAKS) as f:
             return float(json.load(f)["hbm_gbs"]), "measured"
     except Exception:
         return FALLBACK_HBM_GBS, "fallback"
-
-
-def traffic_per_launch():
-    """DRAM bytes per k_step backward launch from the committed ncu summary, if any."""
-    try:
-        with open(TRAFFIC_SUMMARY) as f:
-            for line in f:
-                if line.startswith("traffic_bytes_per_launch_full_size:"):
-                    return float(line.split(":", 1)[1].split()[0])
-    except OSError:
-        pass
-    return None
 
 
 class ClockSampler:
@@ -391,8 +399,9 @@ def compact_line(line):
 
 
 def run_batched(args, eng, rank=0, ws=1):
-    """The batched UQ ensemble through the serving engine: every member resident at once,
-    advanced together by the batched step kernels.  Timed from the first submit (host
+    """The batched UQ ensemble through the serving engine: every member resident at once, its passes
+    run on the chip, small ones sharing a launch (with --batch-autotune, the step kernels advance all
+    of them together).  Timed from the first submit (host
     buffers) to the last image on the host; a sample of the members is also run one at a
     time through the plain path for the served-vs-plain ratio.  With N ranks each runs its
     round-robin share of the members; value = all ranks' cell-updates / the slowest rank's
@@ -438,9 +447,9 @@ def run_batched(args, eng, rank=0, ws=1):
     srv = eng.Server(0, max_members=min(len(inputs), 1024), steps_per_launch=args.steps_per_launch)
     t0 = time.perf_counter()
     ids = [srv.submit(inp[0].replace(tile_x=width[i]), *inp[1:]) for i, inp in enumerate(inputs)]
-    # while every member is in its forward pass (they are admitted together), time whole
-    # batched steps (k_mstep + k_bpsi + k_bstrip) from the server's CUDA events
-    # (and the tile kernel alone on one step per replay, k_mstep, timed by the server)
+    # while every member is in its forward pass (they are admitted together), time whole steps of
+    # all of them from the server's CUDA events (and, with the step kernels, the tile kernel alone on
+    # one step per replay, k_mstep, timed by the server)
     fwd_ms, fwd_steps, calls = 0.0, 0, 0
     tile_ms = []
     out = {}
@@ -452,7 +461,8 @@ def run_batched(args, eng, rank=0, ws=1):
         if calls >= 2 and (calls + 1) * args.steps_per_launch <= nt_min:
             fwd_ms += srv.stats()["gpu_ms"] - ms0
             fwd_steps += args.steps_per_launch
-            tile_ms.append(srv.kernel_ms())
+            if args.batch_autotune:
+                tile_ms.append(srv.kernel_ms())
         r = srv.poll()
         while r is not None:
             out[r[0]] = r[1:]
@@ -464,14 +474,22 @@ def run_batched(args, eng, rank=0, ws=1):
     srv.close()
     step_roof = None
     if fwd_steps:
-        step_bytes = sum(algorithmic_bytes(p)["batched_fwd_step"] for p, *_ in inputs)
-        achieved = step_bytes / (fwd_ms / fwd_steps * 1e-3) / 1e9
-        peak, peak_kind = hbm_peak()
-        step_roof = {"bound": "hbm", "what": "whole batched forward step (k_mstep + k_bpsi + k_bstrip)",
-                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_source": peak_kind, "algorithmic_bytes_per_step": step_bytes,
-                     "ms_per_step": fwd_ms / fwd_steps, "steps_timed": fwd_steps,
-                     "note": "CUDA events around graph replays of the server's stream"}
+        ms = fwd_ms / fwd_steps
+        if args.batch_autotune:
+            step_bytes = sum(algorithmic_bytes(p)["batched_fwd_step"] for p, *_ in inputs)
+            achieved = step_bytes / (ms * 1e-3) / 1e9
+            peak, peak_kind = hbm_peak()
+            step_roof = {"bound": "hbm", "what": "whole batched forward step (k_mstep + k_bpsi + k_bstrip)",
+                         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                         "peak_source": peak_kind, "algorithmic_bytes_per_step": step_bytes}
+        else:
+            flops = sum(flops_per_step(p)[0] for p, *_ in inputs)
+            achieved, peak = flops / (ms * 1e-3) / 1e12, fp32_peak()
+            step_roof = {"bound": "fp32", "what": "one forward step of every member (k_resident, in waves)",
+                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+                         "peak_source": "nominal", "algorithmic_flops_per_step": flops}
+        step_roof.update({"ms_per_step": ms, "steps_timed": fwd_steps,
+                          "note": "CUDA events around the work of the server's steps on its stream"})
     tile_roof = None
     tile_ms = [t for t in tile_ms if t > 0]
     if tile_ms:
@@ -807,7 +825,7 @@ def run_gpu(args):
     p, ext_true, ext, wav = workload(args)
     # observed data: forward modelling on the true model with trace recording (untimed)
     seis = eng.model_seismogram(p.replace(storage=0), ext_true, wav)
-    # step-kernel tile width for this grid shape (plans below use it: tile_x = 0)
+    # step-kernel tile width for this grid shape (what plans of tile_x = 0 fall back to)
     tuned = None
     if not args.tile_x:
         tx, ms = eng.autotune(p, 200)
@@ -827,10 +845,9 @@ def run_gpu(args):
         plan.forward(d_vel, d_wav)
         plan.adjoint(d_seis, d_img, d_slf)
 
-    # Sampled kernel timing (of every 16 steps, 8 consecutive k_step launches bracketed by one
-    # pair of CUDA events on the plan's stream, so that they keep their programmatic overlap)
-    # is switched on before the warm-up, so the time-loop graphs are captured with those
-    # events outside the timed region; the timed migrations replay them.
+    # Sampled kernel timing, switched on before the warm-up: a pair of CUDA events on the plan's stream
+    # around each resident pass (with the step kernels, of every 16 steps around 8 consecutive
+    # launches, captured into the time-loop graphs outside the timed region).
     plan.profile(16)
     torch.cuda.synchronize()
     for _ in range(args.warmup):
@@ -935,19 +952,21 @@ def run_gpu(args):
     nbytes = algorithmic_bytes(p)
     bwd_avg_ms = prof["bwd_ms"] / max(prof["bwd_n"], 1)
     fwd_avg_ms = prof["fwd_ms"] / max(prof["fwd_n"], 1)
-    achieved = nbytes["k_step_bwd"] / (bwd_avg_ms * 1e-3) / 1e9
-    peak, peak_kind = hbm_peak()
-    roofline = {"bound": "hbm", "kernel": "k_step<float,backward>", "achieved": achieved,
-                "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic_per_launch(), "peak_source": peak_kind,
-                "algorithmic_bytes_per_launch": nbytes["k_step_bwd"],
-                "avg_launch_ms": bwd_avg_ms, "sampled_launches": prof["bwd_n"],
-                "fwd_kernel_avg_launch_ms": fwd_avg_ms,
-                "fwd_kernel_achieved_gbs": nbytes["k_step_fwd"] / (fwd_avg_ms * 1e-3) / 1e9,
-                "timing": "CUDA events on the plan's stream around blocks of 8 consecutive launches "
-                          "(of every 16 steps) inside the time-loop graph; avg = block time / launches",
-                "note": "the step kernel updates the CPML psi itself (no separate psi kernel); "
-                        "traffic: cold-cache ncu reads of one launch"}
+    flops_fwd, flops_bwd = flops_per_step(p)
+    peak = fp32_peak()
+    hbm, hbm_kind = hbm_peak()
+    achieved = flops_bwd / (bwd_avg_ms * 1e-3) / 1e12
+    resident = not args.tile_x                           # a forced width takes the step kernels
+    roofline = {"bound": "fp32", "kernel": "k_resident<float> (adjoint)" if resident else "k_step<float,backward>",
+                "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+                "traffic": None, "peak_source": "nominal: SMs x 128 FMA x highest clock",
+                "algorithmic_flops_per_step": flops_bwd, "avg_step_ms": bwd_avg_ms, "steps_timed": prof["bwd_n"],
+                "fwd_avg_step_ms": fwd_avg_ms, "fwd_achieved_tflops": flops_fwd / (fwd_avg_ms * 1e-3) / 1e12,
+                "streaming_equivalent_gbs": nbytes["k_step_bwd"] / (bwd_avg_ms * 1e-3) / 1e9,
+                "hbm_peak_gbs": hbm, "hbm_peak_source": hbm_kind,
+                "timing": "CUDA events on the plan's stream around the pass; avg = its time / steps",
+                "note": "the fields stay in shared and tensor memory over the whole pass; streaming_equivalent "
+                        "is what a kernel that streams them through HBM at every step would have moved"}
     served = None
     if ws == 1 and args.serve_requests > 0:
         cap = batched["value"] if batched else value
