@@ -77,7 +77,8 @@ typedef struct rtm_params {
     int storage;               /* enum rtm_storage                                    */
     int precision;             /* enum rtm_precision (stored source wavefield)        */
     int compute;               /* enum rtm_compute                                    */
-    int tile_x;                /* x columns per CTA tile: 0 = autotuned default        */
+    int tile_x;                /* 0: whole passes on the chip where the grid fits (else the step
+                                  kernels, autotuned); 8, 16, 32: step kernels of that tile width */
     int reserved[3];
 } rtm_params;
 
@@ -195,7 +196,7 @@ int rtm_normalized_cross_correlation(const rtm_params *p, float *image, float *s
  * Times `steps` forward steps of *p's grid shape for every tile width the step kernel
  * supports (8, 16, 32 columns: 4, 8, 16 warps per CTA; FP64 up to 16) and remembers the
  * fastest for that shape (grid, CPML, storage, precision, compute): every plan created
- * afterwards with tile_x = 0 for that shape uses it.  Returns the choice and its time per
+ * afterwards with tile_x = 0 for that shape uses it where its passes run step by step.  Returns the choice and its time per
  * step.  Process-wide, thread-safe.  No counterpart in the reference. */
 int rtm_autotune(const rtm_params *p, int steps, int *best_tile_x, float *ms_per_step);
 
@@ -231,10 +232,10 @@ int rtm_plan_sync(rtm_plan *plan);
 long long rtm_plan_launch_count(const rtm_plan *plan);
 /* Device bytes the plan holds. */
 long long rtm_plan_bytes(const rtm_plan *plan);
-/* Sampled kernel timing: with every > 0, each step whose index is a multiple of `every`
- * brackets its fused step kernel with CUDA events on the plan's stream (0 = off).
- * _read returns the summed milliseconds and launch counts (forward, backward) since the
- * last call and resets them. */
+/* Sampled kernel timing: with every > 0, CUDA events on the plan's stream bracket each pass that
+ * runs on the chip, or, step by step, launches of the step kernel in every `every` steps (0 = off).
+ * _read returns the summed milliseconds and the time steps in them (forward, backward) since
+ * the last call and resets them. */
 int rtm_plan_profile(rtm_plan *plan, int every);
 int rtm_plan_profile_read(rtm_plan *plan, double *fwd_ms, int *fwd_n, double *bwd_ms, int *bwd_n);
 
@@ -246,9 +247,11 @@ void rtm_release_cached(void);
  * run rtm_routine for disjoint simulation ranges, with no messages) by many migrations
  * resident on one GPU.  A server admits submitted migrations (any grid, time axis, storage
  * precision; FP32 compute) in arrival order while a member slot is free and their footprint
- * fits the HBM budget, and advances every resident migration one time step per batched step
- * -- one k_bpsi + one k_bstep launch over a (migration, tile) work list, replayed from a
- * CUDA graph.  Finished migrations free their slots for the next admissions (continuous
+ * fits the HBM budget.  Their passes run on the chip, small grids sharing a launch; each is owed
+ * steps_per_launch time steps a server step, and a quarter of the launches runs at each, for
+ * all the steps its members are owed.  Requests with a forced tile_x, or on grids that do not
+ * fit the chip, advance together, one time step per batched step, by kernels over a (migration,
+ * tile) work list replayed from a CUDA graph.  Finished migrations free their slots for the next admissions (continuous
  * batching).  One thread drives a server. */
 typedef struct rtm_server rtm_server;
 
@@ -260,7 +263,6 @@ int rtm_server_destroy(rtm_server *server);
  * wavelet: n_wavelet, seismogram: rec_count x nt). */
 int rtm_server_submit(rtm_server *server, const rtm_params *p, const float *velocity,
                       const float *wavelet, const float *seismogram, long long *request_id);
-/* Admits, runs steps_per_launch batched steps, harvests finished migrations. */
 /* As rtm_server_submit, with the seismogram as a ZFP fixed-accuracy stream of rec_count x nt
  * (zfp2d_lossyCompression's output, tolerance tol): a host thread of the server decodes it
  * (rtm_zfp_decode_float2d) while the GPU steps, and the request is admitted once decoded;
@@ -268,6 +270,7 @@ int rtm_server_submit(rtm_server *server, const rtm_params *p, const float *velo
 int rtm_server_submit_zfp(rtm_server *server, const rtm_params *p, const float *velocity,
                           const float *wavelet, const void *zfp_stream, size_t zfp_bytes,
                           float tol, long long *request_id);
+/* Admits, advances the active migrations, harvests finished ones. */
 int rtm_server_step(rtm_server *server, int *n_active, int *n_queued);
 /* One finished migration (RTM_ERR_BUSY if none): image and self image (nx x nz, each may be
  * NULL), times[3] = submit, admission, completion (seconds, monotonic clock; may be NULL). */
@@ -289,8 +292,8 @@ int rtm_server_stats(const rtm_server *server, long long *cell_updates, double *
 int rtm_server_kernel_ms(const rtm_server *server, double *tile_kernel_ms);
 /* Tile width of the batched kernel (32 or 16 columns) for p's grid shape, chosen by timing
  * `members` copies of p (nt shortened to `steps`) through a server with each width; later
- * submissions of that shape with tile_x = 0 use it (tile_x = 16 or 32 in a request forces a
- * width).  *best_ms_per_step: the batch's GPU time per batched step at that width.  No
+ * submissions of that shape with tile_x = 0 use it where the batched kernels run them (tile_x =
+ * 16 or 32 in a request forces a width and those kernels).  *best_ms_per_step: the batch's GPU time per batched step at that width.  No
  * counterpart in the reference. */
 int rtm_autotune_batched(const rtm_params *p, int members, int steps, int *best_tile_x,
                          float *best_ms_per_step);
