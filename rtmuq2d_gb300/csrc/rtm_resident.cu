@@ -522,8 +522,9 @@ __device__ __forceinline__ void res_leap(const ResJob<T> &J, const ResCta &c, co
 
 // What stays the same for a thread of a strip block at every step, with NC > 0: its psi quads (a count
 // in the left or right strip and one in the top or bottom one, at a fixed stride of columns) and where
-// the psi of its own quads lies.  Worked out at every step, the index arithmetic and its chain of shared loads took a
-// third of a small grid's step.  (A block that holds both strips of an axis runs with NC = 0.)
+// the psi of its own quads lies.  Worked out at every step, the index arithmetic and its chain of
+// shared loads took a third of a small grid's step.  (A block that holds both strips of an axis runs
+// with NC = 0.)
 // Packed: they live in registers over all steps, and a word spilt costs a way to the second-level
 // cache at every one (offsets are below 65536: 224 KB hold 57344 values).
 struct ResFix {
@@ -989,6 +990,13 @@ __device__ __forceinline__ void ring_item(const Geom &g, const RingBox &b, int i
 }
 
 // A run of steps of one pass on one block.
+// What bounds it: on small grids (NC = 1, 2) a chain of latencies -- the exchange through the second-level
+// cache, psi, leapfrog and strips a quad a thread, two to four barriers; on large ones (NC = 0) the issue
+// slots and shared-memory latency of 16 warps, at the 128 registers that 512 threads leave.  256 threads
+// would leave 255 but half the warps; more than 512 fewer registers than the window alone needs.
+// A forward and a backward step together, step kernels -> here: 96 x 64 17.2 -> 4.7 us, 400 x 200
+// 17.7 -> 5.5, 901 x 301 (FP16 snapshots) 18.3 -> 8.2, 2000 x 600 (snapshots) 25.0 -> 13.5, 3400 x 700
+// 38.9 -> 21.5, 400 x 200 in double 120 -> 39.
 template <typename T, int NC>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_resident(const ResJob<T> *__restrict__ jobs, const ResCta *__restrict__ ctas, unsigned long long *xch, int pt0,
