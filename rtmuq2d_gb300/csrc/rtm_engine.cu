@@ -705,7 +705,11 @@ static ResJob<T> resident_job(rtm_plan *P, int back)
     J.storage = P->p.storage;
     for (int k = 0; k < 2; ++k) { J.u[k] = P->at<T>(P->L.u[k]); J.r[k] = P->at<T>(P->L.r[k]); }
     J.coef = P->at<T>(P->L.coef);
-    for (int k = 0; k < 4; ++k) { J.psi[k] = P->at<T>(P->L.psi[k]); J.xi[k] = P->at<T>(P->L.xi[k]); }
+    for (int k = 0; k < 4; ++k) {
+        J.psi[0][k] = P->at<T>(P->L.psi[k]);
+        J.psi[1][k] = P->at<T>(P->L.psn[k]);
+        J.xi[k] = P->at<T>(P->L.xi[k]);
+    }
     const float *prof = P->at<float>(P->L.prof);
     const ProfLayout pl = prof_layout(g);
     for (int k = 0; k < 8; ++k) J.prof[k] = prof + pl.off[k];

@@ -266,7 +266,8 @@ struct ResJob {
     int storage;
     T *u[2], *r[2];
     const T *coef;
-    T *psi[4], *xi[4];                // left, right, top, bottom: only between the runs of a pass
+    T *psi[2][4], *xi[4];             // left, right, top, bottom: only between the runs of a pass; psi of
+                                      // a run that ends at (starts from) step t in psi[t & 1]
     const float *prof[8];             // a_l b_l a_r b_r a_t b_t a_b b_b
     const int *rec_last, *rec_first, *rec_cnt;
     const float *wav, *seis_t;

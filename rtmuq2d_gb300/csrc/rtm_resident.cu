@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 const int k = i / h.HQ, q = i - k * h.HQ, li = c0 - 4 + k - base;
                 if (li < 0 || li >= (side == 0 ? g.thl : g.thr)) continue;
                 T v4[4];
-                ld4(J.psi[side] + (size_t)li * P + c.za + 4 * q, v4);
+                ld4(J.psi[t0 & 1][side] + (size_t)li * P + c.za + 4 * q, v4);
                 st4(ps + k * h.PH + 4 * q, v4);
             }
         }
@@ -1126,7 +1126,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 const int k = i / nq, z = q0 - 4 + 4 * (i - k * nq);
                 if (z - sh < 0 || z - sh + 4 > st) continue;
                 T v4[4];
-                ld4(J.psi[2 + side] + (size_t)(c.xa + k) * st + (z - sh), v4);
+                ld4(J.psi[t0 & 1][2 + side] + (size_t)(c.xa + k) * st + (z - sh), v4);
                 st4(ps + k * Pp + (z - (q0 - 4)), v4);
             }
         }
@@ -1376,7 +1376,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
         }
     }
 
-    // ---- the fields back to their buffers (and, between the runs of a pass, psi and xi)
+    // ---- the fields back to their buffers (and, between the runs of a pass, psi and xi).  Neighbours load
+    // some of these cells at their start.  After two steps or more they have: an exchange lies between.  A
+    // run of one step has none: it leaves in u and r what a neighbour may still read as it is (the same
+    // values again, or the other buffer's), and its psi goes to the buffer it did not come from.
     if (!dead) {
         if constexpr (NC == 0) tm_wait_st();
         const T *own = su + (th.xk + kResPad) * h.SP + kResPad + 4 * th.q;
@@ -1452,7 +1455,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     const int k = i / h.HQ, q = i - k * h.HQ;
                     T v4[4];
                     ld4(ps + (k + 4) * h.PH + 4 * q, v4);
-                    st4(J.psi[side] + (size_t)(c0 + k - base) * P + c.za + 4 * q, v4);
+                    st4(J.psi[t1 & 1][side] + (size_t)(c0 + k - base) * P + c.za + 4 * q, v4);
                 }
             }
             for (int side = 0; side < 2; ++side) {
@@ -1465,7 +1468,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     const int k = i / nq, z = q0 + 4 * (i - k * nq);
                     T v4[4];
                     ld4(ps + k * Pp + 4 + (z - q0), v4);
-                    st4(J.psi[2 + side] + (size_t)(c.xa + k) * st + (z - sh), v4);
+                    st4(J.psi[t1 & 1][2 + side] + (size_t)(c.xa + k) * st + (z - sh), v4);
                 }
             }
         }
