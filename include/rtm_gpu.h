@@ -248,8 +248,8 @@ void rtm_release_cached(void);
  * resident on one GPU.  A server admits submitted migrations (any grid, time axis, storage
  * precision; FP32 compute) in arrival order while a member slot is free and their footprint
  * fits the HBM budget.  Their passes run on the chip, small grids sharing a launch; each is owed
- * steps_per_launch time steps a server step, and an eighth of the launches runs at each, for
- * all the steps its members are owed.  Requests with a forced tile_x, or on grids that do not
+ * steps_per_launch time steps a server step, and an eighth of the launches runs at each (more
+ * above 64), in turn, for the steps its members are owed, up to 512 at once.  Requests with a forced tile_x, or on grids that do not
  * fit the chip, advance together, one time step per batched step, by kernels over a (migration,
  * tile) work list replayed from a CUDA graph.  Finished migrations free their slots for the next admissions (continuous
  * batching).  One thread drives a server. */

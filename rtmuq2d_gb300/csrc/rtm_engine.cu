@@ -30,6 +30,7 @@
 #include "rtm_gpu.h"
 #include "rtm_internal.h"
 #include "rtm_partition.h"
+#include "rtm_waves.h"
 
 namespace rtm {
 

@@ -69,6 +69,8 @@ struct rtm_server {
     // step, so their launches need no device state
     std::vector<int> res_pass, res_step;
     std::vector<int> res_due;              // steps a member is owed: it gains steps_per_launch a server step
+    std::vector<long long> res_ran;        // step_resident call of its last launch (of its admission before that)
+    long long res_steps = 0;               // step_resident calls
     struct ResKey {
         int dimx, dimz, thl, thr, thu, thd, fields, sms;
         bool operator<(const ResKey &o) const
@@ -175,9 +177,8 @@ static void rebuild_index(rtm_server *S)
 }
 
 // ---- resident members ------------------------------------------------------------------------
-// A server's members run as resident passes where they fit: each rtm_server_step advances every one
-// of them by up to steps_per_launch steps (a launch ends with its member's pass).  Large members take
-// the chip one after the other; small ones share a launch, each with its part of the SMs.
+// A server's members run as resident passes where they fit (a launch ends with its member's pass);
+// rtm_waves.h says which of them run at a server step, and beside which others.
 
 static int res_fields(const rtm_plan *P, int pass) { return pass == 2 && P->p.storage == RTM_STORE_RING ? 2 : 1; }
 
@@ -220,104 +221,23 @@ static int res_room(rtm_server *S, E *&buf, size_t &have, size_t want)
     return RTM_OK;
 }
 
-// A member that shares a launch takes about one SM per kResCells cells, in whole shares of the chip so
-// that a few partitions serve every mix (and more where SMs are spare): the exchange and the strips of
-// a step cost nearly the same whatever a block holds, so the fullest blocks that fit do the most cells a
-// second.  24 mixed members of 400 x 200 to 3400 x 700: 8000 cells an SM 166 ms, 12000 154, 16000 147,
-// 20000 146, and no less with 24000 or 48000 (what does not fit takes a larger share).
-constexpr double kResCells = 20000.0;
-constexpr int kResMostSteps = 512;        // steps of one launch at most
-
-// One server step of the resident members.  Every one of them is owed steps_per_launch steps; of the
-// launches (members that fit beside one another) an eighth runs, those owed most, each for all the
-// steps it is owed: with eight launches or more a member's fields are brought on and off the chip once
-// in eight server steps, for the same progress (12 members of 3400 x 700: 3.5 us of 10 a step went into
-// it at 16 steps a launch).  A quarter: 64 members 213.6 Gcell-updates/s on the GPU against 218.3, 12
-// members 202.6 ms against 200.9; a 32nd 196.5 but 24 mixed ones 146.4 -> 147.8.
+// One server step of the resident members: the launches that res_waves picks.
 static int step_resident(rtm_server *S, bool sampled)
 {
-    struct Item {
-        int m, share;                     // slot; it takes sms / share SMs
-        int t0, t1, back;
-        int lo, hi;                       // 16-bit storage: slots its steps write or read
-    };
-    std::vector<Item> items;
+    using Item = WaveItem;
     if (S->parts.size() >= 256) S->parts.clear();
+    ++S->res_steps;
+    std::vector<WaveMember> members;
     for (int m = 0; m < S->max_members; ++m) {
         const rtm_plan *P = S->slot_plan[m];
         if (!P || S->res_pass[m] < 1 || S->res_pass[m] > 2) continue;
-        const Geom &g = P->g;
-        Item it;
-        it.m = m;
-        it.back = S->res_pass[m] - 1;
-        it.t0 = S->res_step[m];
-        S->res_due[m] = std::min(S->res_due[m] + S->steps_per_launch, kResMostSteps);
-        it.t1 = std::min(g.nt, it.t0 + S->res_due[m]);
-        it.lo = 0;
-        it.hi = -1;
-        if (P->p.precision != RTM_PREC_FP32) {
-            const int nt = g.nt, sl = g.slices;
-            if (P->p.storage == RTM_STORE_RING) {
-                it.lo = it.back ? nt - it.t1 + 1 : it.t0 + 1;
-                it.hi = it.back ? nt - std::max(it.t0 - 1, 2) : std::min(it.t1, nt - 1);
-            } else {
-                it.lo = (it.back ? nt - it.t1 + sl - 1 : it.t0 + sl - 1) / sl;
-                it.hi = it.back ? (nt - 1 - it.t0) / sl : (it.t1 - 1) / sl;
-            }
-        }
-        const int want = std::max(1, (int)((double)g.dimx * g.dimz / kResCells + 0.999));
-        it.share = std::max(1, std::min(S->sms / want, 16));
-        while (it.share > 1 && !res_part(S, P, it.back + 1, S->sms / it.share)) --it.share;
-        items.push_back(it);
+        S->res_due[m] = wave_owe(S->res_due[m], S->steps_per_launch);
+        members.push_back({m, &P->g, S->res_pass[m] - 1, S->res_step[m], S->res_due[m], S->res_ran[m], P->p.precision, P->p.storage});
     }
-    std::stable_sort(items.begin(), items.end(), [](const Item &a, const Item &b) { return a.share < b.share; });
-    auto part_of = [&](const Item &it) { return res_part(S, S->slot_plan[it.m], it.back + 1, S->sms / it.share); };
-
-    // ---- the launches: the largest member left and those that fit beside it
-    std::vector<std::vector<Item>> waves;
-    std::vector<char> taken(items.size(), 0);
-    for (size_t first = 0; first < items.size(); ++first) {
-        if (taken[first]) continue;
-        std::vector<Item> wave;
-        int used = 0;
-        for (size_t i = first; i < items.size(); ++i) {
-            const int need = S->sms / items[i].share;
-            if (taken[i] || used + need > S->sms) continue;
-            taken[i] = 1;
-            used += need;
-            wave.push_back(items[i]);
-        }
-        // spare SMs to the member with the most cells an SM, which the others wait for, as long as there
-        // are enough (four members of 400 x 200, 1000 steps a pass: 20 ms, 33 where the first took all it could)
-        std::vector<int> share(wave.size());
-        for (size_t i = 0; i < wave.size(); ++i) share[i] = wave[i].share;
-        for (;;) {
-            size_t slow = 0;
-            double most = -1.0;
-            for (size_t i = 0; i < wave.size(); ++i) {
-                const Geom &g = S->slot_plan[wave[i].m]->g;
-                const double per = (double)g.dimx * g.dimz / (S->sms / share[i]);
-                if (per > most) { most = per; slow = i; }
-            }
-            if (share[slow] == 1) break;
-            const int more = S->sms / (share[slow] - 1) - S->sms / share[slow];
-            if (used + more > S->sms) break;
-            used += more;
-            --share[slow];
-        }
-        for (size_t i = 0; i < wave.size(); ++i)
-            if (res_part(S, S->slot_plan[wave[i].m], wave[i].back + 1, S->sms / share[i])) wave[i].share = share[i];
-        waves.push_back(std::move(wave));
-    }
+    const auto waves = res_waves(members, S->sms, S->steps_per_launch,
+                                 [&](int m, int back, int sms) { return res_part(S, S->slot_plan[m], back + 1, sms); });
     if (waves.empty()) return RTM_OK;
-    auto due_of = [&](const std::vector<Item> &w) {
-        int d = 0;
-        for (const Item &it : w) d = std::max(d, S->res_due[it.m]);
-        return d;
-    };
-    std::stable_sort(waves.begin(), waves.end(),
-                     [&](const std::vector<Item> &a, const std::vector<Item> &b) { return due_of(a) > due_of(b); });
-    waves.resize((waves.size() + 7) / 8);
+    auto part_of = [&](const Item &it) { return res_part(S, S->slot_plan[it.m], it.back + 1, S->sms / it.share); };
     size_t xch = 0, stage = 0;
     for (const auto &wave : waves) {
         size_t wx = 0, ws = 0;
@@ -421,6 +341,7 @@ static int step_resident(rtm_server *S, bool sampled)
             S->res_due[it.m] -= it.t1 - it.t0;
             if (it.t1 == S->slot_plan[it.m]->g.nt) S->res_due[it.m] = 0;     // (the next pass starts afresh)
             S->res_step[it.m] = it.t1;
+            S->res_ran[it.m] = S->res_steps;
         }
     }
     return RTM_OK;
@@ -490,6 +411,7 @@ static int admit(rtm_server *S, int m, ServeRequest *R)
     S->res_pass[m] = res_member(S, P, R) ? -1 : 0;       // resident from its activation on
     S->res_step[m] = 0;
     S->res_due[m] = 0;
+    S->res_ran[m] = S->res_steps;
     R->t_admit = now_s();
     return RTM_OK;
 }
@@ -651,6 +573,7 @@ static int server_init(rtm_server *S, long long hbm_budget_bytes)
     S->res_pass.assign(S->max_members, 0);
     S->res_step.assign(S->max_members, 0);
     S->res_due.assign(S->max_members, 0);
+    S->res_ran.assign(S->max_members, 0);
     {
         int dev = 0, coop = 0;
         RTM_CUDA(cudaGetDevice(&dev));

@@ -43,3 +43,24 @@ def test_launches_of_a_step_or_a_few(engine, case, steps_per_launch):
     want = engine.migrate_shot(*r)
     assert np.abs(want[0]).max() > 0
     assert np.array_equal(img, want[0]) and np.array_equal(slf, want[1])
+
+
+def test_members_share_the_steps_at_large_launches(engine):
+    """Three members that fill the chip, 256 steps a launch: they finish within a few server steps of one
+    another, each with the image of its own uncut migration."""
+    rs = [_request(engine, 2600, 600, (50, 50, 50, 50), 4000, 40, k) for k in range(3)]
+    srv = engine.Server(0, max_members=8, steps_per_launch=256)
+    ids = [srv.submit(*r) for r in rs]
+    done, at, step = {}, {}, 0
+    while len(done) < len(ids):
+        srv.step()
+        step += 1
+        assert step < 60
+        while (r := srv.poll()) is not None:
+            done[r[0]], at[r[0]] = r[1:3], step
+    srv.close()
+    # two of the three waves run at a server step, so a turn takes two; admissions may lie two steps apart
+    assert max(at.values()) - min(at.values()) <= 4, at
+    for i, r in zip(ids, rs):
+        want = engine.migrate_shot(*r)
+        assert np.array_equal(done[i][0], want[0]) and np.array_equal(done[i][1], want[1])
