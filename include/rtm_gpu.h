@@ -255,7 +255,12 @@ void rtm_release_cached(void);
  * batching).  One thread drives a server. */
 typedef struct rtm_server rtm_server;
 
-/* hbm_budget_bytes <= 0: 80 % of the free device memory.  max_members <= 1024. */
+/* hbm_budget_bytes <= 0: 80 % of the free device memory.  max_members <= 1024.  The budget holds
+ * the members' buffers (rtm_footprint_bytes each) and what the launches of passes on the chip need:
+ * their tables, mailboxes (27 MB, or what the members' grids take where that is too much) and, for
+ * 16-bit storage, full-precision slots of the steps of a launch (at most a 64th of the budget, or
+ * 128 MB if that is more; a launch takes as many steps as they hold).  A member for which that does
+ * not fit runs with the kernels over a work list. */
 int rtm_server_create(long long hbm_budget_bytes, int max_members, int steps_per_launch,
                       rtm_server **server);
 int rtm_server_destroy(rtm_server *server);

@@ -82,10 +82,10 @@ struct rtm_server {
     std::map<ResKey, rtm::ResPart> parts;  // blocks per grid shape and SM share (bounded: cleared at 256)
     rtm::ResJob<float> *d_jobs = nullptr;
     rtm::ResCta *d_ctas = nullptr;
-    unsigned long long *d_xch = nullptr;   // exchange buffer of the largest launch so far
+    unsigned long long *d_xch = nullptr;   // exchange buffer of a launch
     float *d_stage16 = nullptr;            // full-precision slots of the 16-bit members of a launch
-    size_t job_room = 0, cta_room = 0, xch_room = 0, stage16_room = 0;   // elements
-    unsigned res_tag = 1;
+    size_t job_room = 0, cta_room = 0, xch_room = 0, stage16_room = 0;   // elements; their bytes are in in_use
+    unsigned res_tag = 0;                  // tag of the next launch's first step; 0: the exchange buffer is not zeroed yet
     int res_sampled = 0;                   // steps of the resident launch between kev0 and kev1
     int sms = 0;
     // host threads decoding ZFP seismograms of submitted requests (rtm_server_submit_zfp)
@@ -196,29 +196,98 @@ static const ResPart *res_part(rtm_server *S, const rtm_plan *P, int pass, int s
     return it->second.ctas.empty() ? nullptr : &it->second;
 }
 
-// Whether a request runs resident: no batched tile width asked for, and both passes fit the chip.
+// Drops plans kept for reuse until `bytes` more fit the budget, or none is left.
+static void make_room(rtm_server *S, long long bytes)
+{
+    while (!S->idle.empty() && S->in_use + bytes > S->budget) {
+        S->in_use -= (long long)S->idle.back()->L.total;
+        plan_free(S->idle.back());
+        S->idle.pop_back();
+    }
+}
+
+// Grows a buffer of the resident members to `want` elements, within the budget (the old one counted until
+// it is gone); it stays as it is when there is no room (false).
+template <typename E>
+static bool res_room(rtm_server *S, E *&buf, size_t &have, size_t want)
+{
+    if (have >= want) return true;
+    E *grown = nullptr;
+    if (S->in_use + (long long)(want * sizeof(E)) > S->budget) return false;
+    if (cudaMalloc(&grown, want * sizeof(E)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (buf) {
+        cudaStreamSynchronize(S->stream);
+        cudaFree(buf);
+    }
+    S->in_use += (long long)((want - have) * sizeof(E));
+    buf = grown;
+    have = want;
+    return true;
+}
+
+static long long res_room_bytes(const rtm_server *S)
+{
+    return (long long)(S->job_room * sizeof(ResJob<float>) + S->cta_room * sizeof(ResCta) +
+                       S->xch_room * sizeof(unsigned long long) + S->stage16_room * sizeof(float));
+}
+
+static bool any_resident(const rtm_server *S)
+{
+    for (int m = 0; m < S->max_members; ++m)
+        if (S->slot_plan[m] && S->res_pass[m] != 0) return true;
+    return false;
+}
+
+// Gives the resident members' buffers back (none of them is admitted).
+static void res_release(rtm_server *S)
+{
+    cudaStreamSynchronize(S->stream);
+    S->in_use -= res_room_bytes(S);
+    cudaFree(S->d_jobs); cudaFree(S->d_ctas); cudaFree(S->d_xch); cudaFree(S->d_stage16);
+    S->d_jobs = nullptr; S->d_ctas = nullptr; S->d_xch = nullptr; S->d_stage16 = nullptr;
+    S->job_room = S->cta_room = S->xch_room = S->stage16_room = 0;
+}
+
+// The exchange buffer at `words` words.  Words that no launch has written carry no step's tag.
+static bool res_xch_room(rtm_server *S, size_t words)
+{
+    if (S->xch_room >= words) return true;
+    if (!res_room(S, S->d_xch, S->xch_room, words)) return false;
+    S->res_tag = 0;                       // zeroed before the next launch
+    return true;
+}
+
+// Whether a request runs resident: no batched tile width asked for, both passes fit the chip, and device
+// memory and the budget hold what its launches need (the tables of every wave of a server step, its
+// mailboxes -- the fullest launch's if they can be had -- and the 16-bit slots of one step).
 static bool res_member(rtm_server *S, const rtm_plan *P, const ServeRequest *R)
 {
     if (R->forced_tile || S->sms < 1 || !resident_wanted(P, true)) return false;
-    return res_part(S, P, 1, S->sms) && res_part(S, P, 2, S->sms);
+    const ResPart *a = res_part(S, P, 1, S->sms), *b = a ? res_part(S, P, 2, S->sms) : nullptr;
+    if (!a || !b) return false;
+    const size_t quads = std::max(a->xch_quads, b->xch_quads);
+    const size_t waves = std::max(((size_t)S->max_members + 7) / 8,
+                                  ((size_t)S->max_members * S->steps_per_launch + kResMostSteps - 1) / kResMostSteps);
+    const size_t stage = wave_least_stage(P->p.precision, P->p.storage, P->L.slot_elems);
+    const size_t fullest = (size_t)S->sms * kResMostXchQuads;
+    if (S->xch_room == 0)
+        make_room(S, (long long)(S->max_members * sizeof(ResJob<float>) + waves * S->sms * sizeof(ResCta) +
+                                 fullest * kXchWords * sizeof(unsigned long long) + stage * sizeof(float)));
+    const bool ok = res_room(S, S->d_jobs, S->job_room, (size_t)S->max_members) && res_room(S, S->d_ctas, S->cta_room, waves * S->sms) &&
+                    (res_xch_room(S, fullest * kXchWords) || res_xch_room(S, quads * kXchWords)) &&
+                    res_room(S, S->d_stage16, S->stage16_room, stage);
+    if (!ok && !any_resident(S)) res_release(S);
+    return ok;
 }
 
-// Device room for `want` elements (grown by a quarter; the stream is idle while it grows).
-template <typename E>
-static int res_room(rtm_server *S, E *&buf, size_t &have, size_t want)
+// Elements that the staging area may grow to: a 64th of the budget, 128 MB at least, within the budget.
+static size_t res_stage_most(const rtm_server *S)
 {
-    if (have >= want) return RTM_OK;
-    RTM_CUDA(cudaStreamSynchronize(S->stream));
-    if (buf) cudaFree(buf);
-    buf = nullptr;
-    have = 0;
-    want += want / 4;
-    if (cudaMalloc(&buf, want * sizeof(E)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(RTM_ERR_NOMEM, "%zu bytes for the resident members", want * sizeof(E));
-    }
-    have = want;
-    return RTM_OK;
+    const long long cap = std::max(S->budget / 64, 128LL << 20), left = std::max(0LL, S->budget - S->in_use);
+    return std::max(S->stage16_room, (size_t)std::min(cap, left) / sizeof(float));
 }
 
 // One server step of the resident members: the launches that res_waves picks.
@@ -232,32 +301,34 @@ static int step_resident(rtm_server *S, bool sampled)
         const rtm_plan *P = S->slot_plan[m];
         if (!P || S->res_pass[m] < 1 || S->res_pass[m] > 2) continue;
         S->res_due[m] = wave_owe(S->res_due[m], S->steps_per_launch);
-        members.push_back({m, &P->g, S->res_pass[m] - 1, S->res_step[m], S->res_due[m], S->res_ran[m], P->p.precision, P->p.storage});
+        members.push_back({m, &P->g, S->res_pass[m] - 1, S->res_step[m], S->res_due[m], S->res_ran[m], P->p.precision,
+                           P->p.storage, P->L.slot_elems});
     }
-    const auto waves = res_waves(members, S->sms, S->steps_per_launch,
-                                 [&](int m, int back, int sms) { return res_part(S, S->slot_plan[m], back + 1, sms); });
-    if (waves.empty()) return RTM_OK;
+    if (members.empty()) return RTM_OK;
+    auto pick = [&](size_t stage_elems) {
+        return res_waves(members, S->sms, S->steps_per_launch, {S->xch_room / kXchWords, stage_elems},
+                         [&](int m, int back, int sms) { return res_part(S, S->slot_plan[m], back + 1, sms); });
+    };
     auto part_of = [&](const Item &it) { return res_part(S, S->slot_plan[it.m], it.back + 1, S->sms / it.share); };
-    size_t xch = 0, stage = 0;
+    const size_t most = res_stage_most(S);
+    auto waves = pick(most);
+    size_t stage = 0;
     for (const auto &wave : waves) {
-        size_t wx = 0, ws = 0;
-        for (const Item &it : wave) {
-            wx += part_of(it)->xch_quads;
+        size_t ws = 0;
+        for (const Item &it : wave)
             if (it.hi >= it.lo) ws += (size_t)(it.hi - it.lo + 1) * S->slot_plan[it.m]->L.slot_elems;
-        }
-        xch = std::max(xch, wx);
         stage = std::max(stage, ws);
     }
-
-    // ---- room, and the tables of all launches in one copy each
-    const size_t words = xch * kXchWords;
-    const bool grown = S->xch_room < words;
-    RTM_TRY(res_room(S, S->d_xch, S->xch_room, words));
-    if (grown || S->res_tag > 0xffffffffu - (unsigned)waves.size() * (kResMostSteps + 2u) - 8u) {
+    // staging for their slots and a quarter more, else shorter runs in the staging there is
+    if (!res_room(S, S->d_stage16, S->stage16_room, std::min(most, stage + stage / 4)) &&
+        !res_room(S, S->d_stage16, S->stage16_room, stage))
+        waves = pick(S->stage16_room);
+    if (S->res_tag == 0 || S->res_tag > 0xffffffffu - (unsigned)waves.size() * (kResMostSteps + 2u) - 8u) {
         RTM_CUDA(cudaMemsetAsync(S->d_xch, 0, S->xch_room * sizeof(unsigned long long), S->stream));
         S->res_tag = 1;
     }
-    RTM_TRY(res_room(S, S->d_stage16, S->stage16_room, stage));
+
+    // ---- the tables of all launches in one copy each
     std::vector<ResJob<float>> jobs;
     std::vector<ResCta> ctas;
     std::vector<size_t> wave_ctas;
@@ -284,8 +355,8 @@ static int step_resident(rtm_server *S, bool sampled)
         }
     }
     wave_ctas.push_back(ctas.size());
-    RTM_TRY(res_room(S, S->d_jobs, S->job_room, jobs.size()));
-    RTM_TRY(res_room(S, S->d_ctas, S->cta_room, ctas.size()));
+    if (jobs.size() > S->job_room || ctas.size() > S->cta_room)      // (reserved for the most waves there can be)
+        return fail(RTM_ERR_STATE, "resident tables: %zu jobs, %zu blocks", jobs.size(), ctas.size());
     // pageable sources: the copies have read them when they return
     RTM_CUDA(cudaMemcpyAsync(S->d_jobs, jobs.data(), jobs.size() * sizeof(ResJob<float>), cudaMemcpyHostToDevice, S->stream));
     RTM_CUDA(cudaMemcpyAsync(S->d_ctas, ctas.data(), ctas.size() * sizeof(ResCta), cudaMemcpyHostToDevice, S->stream));
@@ -362,12 +433,7 @@ static int admit(rtm_server *S, int m, ServeRequest *R)
             break;
         }
     if (!P) {
-        // make room: drop reusable plans that do not match
-        while (!S->idle.empty() && S->in_use + R->bytes > S->budget) {
-            S->in_use -= (long long)S->idle.back()->L.total;
-            plan_free(S->idle.back());
-            S->idle.pop_back();
-        }
+        make_room(S, R->bytes);           // at the cost of reusable plans that do not match
         RTM_TRY(plan_alloc(R->p, &P, true));
         S->in_use += (long long)P->L.total;
         RTM_CUDA(cudaStreamSynchronize(P->stream));
@@ -408,7 +474,8 @@ static int admit(rtm_server *S, int m, ServeRequest *R)
     S->pending.push_back(m);
     S->slot_plan[m] = P;
     S->slot_req[m] = R;
-    S->res_pass[m] = res_member(S, P, R) ? -1 : 0;       // resident from its activation on
+    S->res_pass[m] = 0;
+    if (res_member(S, P, R)) S->res_pass[m] = -1;        // resident from its activation on
     S->res_step[m] = 0;
     S->res_due[m] = 0;
     S->res_ran[m] = S->res_steps;
@@ -770,7 +837,12 @@ int rtm_server_step(rtm_server *S, int *n_active, int *n_queued)
         for (rtm_plan *P : S->idle) if (same_params(P->p, R->p)) reusable = true;
         long long idle_bytes = 0;
         for (rtm_plan *P : S->idle) idle_bytes += (long long)P->L.total;
-        if (!reusable && S->in_use - idle_bytes + R->bytes > S->budget) break;
+        if (!reusable && S->in_use - idle_bytes + R->bytes > S->budget) {
+            // the resident members' buffers outlive them: back with them when a request needs the room
+            if (any_resident(S) || res_room_bytes(S) == 0) break;
+            res_release(S);
+            if (S->in_use - idle_bytes + R->bytes > S->budget) break;
+        }
         const int st = admit(S, slot, R);
         if (st != RTM_OK) return st;
         it = S->queue.erase(it);

@@ -64,3 +64,55 @@ def test_members_share_the_steps_at_large_launches(engine):
     for i, r in zip(ids, rs):
         want = engine.migrate_shot(*r)
         assert np.array_equal(done[i][0], want[0]) and np.array_equal(done[i][1], want[1])
+
+
+def _peak_serve(engine, requests, budget, steps_per_launch=64):
+    """Results, the most bytes the server said it held and the most device memory it took."""
+    import torch
+    torch.cuda.synchronize()
+    free, held, taken = torch.cuda.mem_get_info()[0], 0, 0
+    srv = engine.Server(budget, max_members=8, steps_per_launch=steps_per_launch)
+    base = free - torch.cuda.mem_get_info()[0]             # what every server takes, of any budget
+    ids, out, steps = [srv.submit(*r) for r in requests], {}, 0
+    while len(out) < len(ids):
+        srv.step()
+        steps += 1
+        assert steps < 20000
+        held = max(held, srv.stats()["bytes_in_use"])
+        taken = max(taken, free - torch.cuda.mem_get_info()[0] - base)
+        while (r := srv.poll()) is not None:
+            out[r[0]] = r[1:3]
+    srv.close()
+    return [out[i] for i in ids], held, taken
+
+
+@pytest.mark.parametrize("storage", (0, 1))
+def test_sixteen_bit_members_stay_within_the_budget(engine, storage):
+    """16-bit members whose launches would stage far more than the budget leaves: shorter runs of steps, the
+    device memory within the budget, and the images of a server with all the room, bit for bit."""
+    rs = [_request(engine, 800, 300, (40, 40, 40, 40), 256, 1, k, storage=storage, precision=1 + k % 2) for k in range(2)]
+    want, _, _ = _peak_serve(engine, rs, 0, 256)
+    fp = max(engine.footprint_bytes(r[0]) for r in rs)
+    slack = 8 << 20                                        # allocations are rounded up to 2 MB pages
+    for extra in (64 << 20, 34 << 20):
+        got, held, taken = _peak_serve(engine, rs[:1], fp + extra, 256)
+        assert held <= fp + extra and taken <= fp + extra + slack, (held, taken, fp + extra)
+        assert np.array_equal(got[0][0], want[0][0]) and np.array_equal(got[0][1], want[0][1])
+
+
+def test_members_without_room_for_resident_launches(engine):
+    """A budget that holds a member but not what its resident launches need: the member still runs, and a
+    large request is admitted after resident members although their buffers were in its way."""
+    small = _request(engine, 200, 100, (40, 40, 40, 40), 60, 4, 1)
+    big = _request(engine, 900, 400, (40, 40, 40, 40), 400, 4, 2, storage=0)
+    fps, fpb = engine.footprint_bytes(small[0]), engine.footprint_bytes(big[0])
+    assert fpb > (40 << 20) + fps
+    (got,), held, _ = _peak_serve(engine, [small], fps + (64 << 10))
+    assert held <= fps + (64 << 10)
+    want = engine.migrate_shot(*small)
+    assert np.linalg.norm(got[0].astype(np.float64) - want[0]) <= 1e-5 * np.linalg.norm(want[0])
+    (a, b, c), held, _ = _peak_serve(engine, [small, big, small], fpb + (64 << 10))
+    assert held <= fpb + (64 << 10)
+    assert np.array_equal(a[0], want[0]) and np.array_equal(c[0], want[0])
+    want = engine.migrate_shot(*big)
+    assert np.linalg.norm(b[0].astype(np.float64) - want[0]) <= 1e-5 * np.linalg.norm(want[0])
