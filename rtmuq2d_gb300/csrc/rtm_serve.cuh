@@ -71,15 +71,7 @@ struct rtm_server {
     std::vector<int> res_due;              // steps a member is owed: it gains steps_per_launch a server step
     std::vector<long long> res_ran;        // step_resident call of its last launch (of its admission before that)
     long long res_steps = 0;               // step_resident calls
-    struct ResKey {
-        int dimx, dimz, thl, thr, thu, thd, fields, sms;
-        bool operator<(const ResKey &o) const
-        {
-            return std::tie(dimx, dimz, thl, thr, thu, thd, fields, sms) <
-                   std::tie(o.dimx, o.dimz, o.thl, o.thr, o.thu, o.thd, o.fields, o.sms);
-        }
-    };
-    std::map<ResKey, rtm::ResPart> parts;  // blocks per grid shape and SM share (bounded: cleared at 256)
+    rtm::ResPartCache parts;               // blocks per grid shape and SM share
     rtm::ResJob<float> *d_jobs = nullptr;
     rtm::ResCta *d_ctas = nullptr;
     unsigned long long *d_xch = nullptr;   // exchange buffer of a launch
@@ -185,15 +177,7 @@ static int res_fields(const rtm_plan *P, int pass) { return pass == 2 && P->p.st
 // Blocks of a member's steps of `pass` on `sms` SMs; NULL when they do not fit.
 static const ResPart *res_part(rtm_server *S, const rtm_plan *P, int pass, int sms)
 {
-    const Geom &g = P->g;
-    const rtm_server::ResKey key{g.dimx, g.dimz, g.thl, g.thr, g.thu, g.thd, res_fields(P, pass), sms};
-    auto it = S->parts.find(key);
-    if (it == S->parts.end()) {
-        ResPart part;
-        if (!res_partition(g, key.fields, 4, sms, part)) part = ResPart();
-        it = S->parts.emplace(key, std::move(part)).first;
-    }
-    return it->second.ctas.empty() ? nullptr : &it->second;
+    return S->parts.get(P->g, res_fields(P, pass), sms);
 }
 
 // Drops plans kept for reuse until `bytes` more fit the budget, or none is left.
@@ -260,15 +244,21 @@ static bool res_xch_room(rtm_server *S, size_t words)
     return true;
 }
 
-// Whether a request runs resident: no batched tile width asked for, both passes fit the chip, and device
+// Whether a request runs resident: no batched tile width asked for, both passes fit their share of the chip, and device
 // memory and the budget hold what its launches need (the tables of every wave of a server step, its
 // mailboxes -- the fullest launch's if they can be had -- and the 16-bit slots of one step).
 static bool res_member(rtm_server *S, const rtm_plan *P, const ServeRequest *R)
 {
     if (R->forced_tile || S->sms < 1 || !resident_wanted(P, true)) return false;
-    const ResPart *a = res_part(S, P, 1, S->sms), *b = a ? res_part(S, P, 2, S->sms) : nullptr;
-    if (!a || !b) return false;
-    const size_t quads = std::max(a->xch_quads, b->xch_quads);
+    // the blocks its waves will use, no others: every search takes host time that admission waits for (400
+    // members of different grids 933 -> 793 ms without those for the whole chip)
+    size_t quads = 0;
+    for (int pass = 1; pass <= 2; ++pass) {
+        const int share = wave_share(P->g, S->sms, [&](int s) { return res_part(S, P, pass, S->sms / s) != nullptr; });
+        const ResPart *part = res_part(S, P, pass, S->sms / share);
+        if (!part) return false;
+        quads = std::max(quads, part->xch_quads);
+    }
     const size_t waves = std::max(((size_t)S->max_members + 7) / 8,
                                   ((size_t)S->max_members * S->steps_per_launch + kResMostSteps - 1) / kResMostSteps);
     const size_t stage = wave_least_stage(P->p.precision, P->p.storage, P->L.slot_elems);
@@ -294,7 +284,7 @@ static size_t res_stage_most(const rtm_server *S)
 static int step_resident(rtm_server *S, bool sampled)
 {
     using Item = WaveItem;
-    if (S->parts.size() >= 256) S->parts.clear();
+    S->parts.step();
     ++S->res_steps;
     std::vector<WaveMember> members;
     for (int m = 0; m < S->max_members; ++m) {

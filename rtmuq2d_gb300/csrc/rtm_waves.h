@@ -81,11 +81,22 @@ inline size_t wave_least_stage(int precision, int storage, size_t slot_elems)
     return precision == RTM_PREC_FP32 ? 0 : (storage == RTM_STORE_RING ? 2 : 1) * slot_elems;
 }
 
+// The share of the chip that a member asks for in a wave: its grid's, or the smallest larger one that
+// fits(share) holds for; the whole chip (1) if none does.
+template <typename F>
+int wave_share(const Geom &g, int sms, F fits)
+{
+    const int want = std::max(1, (int)((double)g.dimx * g.dimz / kResCells + 0.999));
+    int share = std::max(1, std::min(sms / want, 16));
+    while (share > 1 && !fits(share)) --share;
+    return share;
+}
+
 // The waves that run at this server step, in order.  part(m, back, sms): the blocks of a pass of member m
-// on that many SMs, NULL when they do not fit.  Every member's blocks fit the whole chip, and the room of a
-// wave holds their mailboxes and one step's staging; members join a wave while it holds theirs, and a wave's
-// 16-bit members take as many steps as it holds slots for (a member of 3400 x 700 with snapshots at every
-// step takes 11 MB a step).
+// on that many SMs, NULL when they do not fit.  Every member's blocks fit at its share (wave_share), and the
+// room of a wave holds their mailboxes and one step's staging; members join a wave while it holds theirs, and
+// a wave's 16-bit members take as many steps as it holds slots for (a member of 3400 x 700 with snapshots at
+// every step takes 11 MB a step).
 // An eighth: 12 members of 3400 x 700 spent 3.5 us of 10 a step on bringing fields on and off the chip at
 // 16 steps a launch.  A quarter: 64 members 213.6 Gcell-updates/s on the GPU against 218.3, 12 members
 // 202.6 ms against 200.9; a 32nd 196.5 but 24 mixed ones 146.4 -> 147.8.
@@ -108,9 +119,7 @@ std::vector<std::vector<WaveItem>> res_waves(const std::vector<WaveMember> &memb
         it.ran = w.ran;
         it.t1 = std::min(w.g->nt, it.t0 + std::min(w.due, kResMostSteps));
         wave_slots(w, it);
-        const int want = std::max(1, (int)((double)w.g->dimx * w.g->dimz / kResCells + 0.999));
-        it.share = std::max(1, std::min(sms / want, 16));
-        while (it.share > 1 && !fits(it, it.share)) --it.share;
+        it.share = wave_share(*w.g, sms, [&](int share) { return fits(it, share); });
         if (w.m >= (int)of.size()) of.resize(w.m + 1);
         of[w.m] = &w;
         items.push_back(it);

@@ -5,8 +5,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <tuple>
 
 #include "rtm_waves.h"
 
@@ -24,18 +22,8 @@ static Geom geom(int nx, int nz, int th, int nt)
     return g;
 }
 
-static std::map<std::tuple<int, int, int, int, int>, ResPart> parts;
-static const ResPart *part_of(const Geom &g, int fields, int sms)
-{
-    auto key = std::make_tuple(g.dimx, g.dimz, g.thl, fields, sms);
-    auto it = parts.find(key);
-    if (it == parts.end()) {
-        ResPart p;
-        if (!res_partition(g, fields, 4, sms, p)) p = ResPart();
-        it = parts.emplace(key, p).first;
-    }
-    return it->second.ctas.empty() ? nullptr : &it->second;
-}
+static ResPartCache parts;
+static const ResPart *part_of(const Geom &g, int fields, int sms) { return parts.get(g, fields, sms); }
 
 // Slots of the store that steps [t0, t1) of a pass write or read, from the kernel's own use of them.
 static bool slot_used(const WaveMember &w, int t0, int t1, int slot)
@@ -161,6 +149,19 @@ int main()
             if (run("16-bit", half, spl, 60, 152, {most * std::min<size_t>(k, 3), least * k})) return 1;
             ++runs;
         }
+    // partitions: what hundreds of members of different grids use is searched for once, and goes once they have
+    ResPartCache c;
+    for (int k = 0; k < 80; ++k) {
+        c.step();
+        for (int m = 0; m < 300; ++m)
+            for (int f = 1; f <= 2; ++f) c.get(geom(64 + m, 48, 16, 8), f, 8);
+    }
+    if (c.searches() != 600) { printf("%lld partitions searched for 600\n", c.searches()); return 1; }
+    for (int k = 0; k < 2 * kResKeepSteps + 1; ++k) {
+        c.step();
+        c.get(geom(64, 48, 16, 8), 1, 8);
+    }
+    if (c.size() > kResKeepParts) { printf("%zu partitions kept of grids long gone\n", c.size()); return 1; }
     printf("ok %d\n", runs);
     return 0;
 }
