@@ -88,7 +88,9 @@ void rtm_params_defaults(rtm_params *p);
  * the grid, nt multiple of time_slices, shot inside the reconstruction region for
  * RTM_STORE_RING). */
 int rtm_params_check(const rtm_params *p);
-/* Device bytes one migration of *p holds (admission by HBM footprint). */
+/* Device bytes of one migration's own buffers (admission by HBM footprint).  A plan whose passes run
+ * on the chip also holds their tables, mailboxes and, for 16-bit storage, full-precision slots, where
+ * device memory has the room: rtm_plan_bytes. */
 long long rtm_footprint_bytes(const rtm_params *p);
 
 const char *rtm_status_string(int status);
@@ -230,7 +232,7 @@ int rtm_plan_capture_source(rtm_plan *plan, int count, const int *times, void *d
 int rtm_plan_sync(rtm_plan *plan);
 /* Number of kernels the plan launched since creation (launch accounting). */
 long long rtm_plan_launch_count(const rtm_plan *plan);
-/* Device bytes the plan holds. */
+/* Device bytes the plan holds, those for passes on the chip included. */
 long long rtm_plan_bytes(const rtm_plan *plan);
 /* Sampled kernel timing: with every > 0, CUDA events on the plan's stream bracket each pass that
  * runs on the chip, or, step by step, launches of the step kernel in every `every` steps (0 = off).

@@ -1430,7 +1430,7 @@ int rtm_plan_profile_read(rtm_plan *plan, double *fwd_ms, int *fwd_n, double *bw
     return RTM_OK;
 }
 
-long long rtm_plan_bytes(const rtm_plan *plan) { return plan ? (long long)plan->L.total : -1; }
+long long rtm_plan_bytes(const rtm_plan *plan) { return plan ? (long long)(plan->L.total + plan->res_bytes) : -1; }
 
 // ---- reference-shaped host-buffer entry points ------------------------------------------
 static rtm_params with_shot(const rtm_params *p, const int *shot)

@@ -116,3 +116,23 @@ def test_members_without_room_for_resident_launches(engine):
     assert np.array_equal(a[0], want[0]) and np.array_equal(c[0], want[0])
     want = engine.migrate_shot(*big)
     assert np.linalg.norm(b[0].astype(np.float64) - want[0]) <= 1e-5 * np.linalg.norm(want[0])
+
+
+@pytest.mark.parametrize("kw", ({}, dict(storage=0, precision=2), dict(precision=1), dict(compute=1), dict(tile_x=16)))
+def test_plan_bytes_are_what_it_takes(engine, kw):
+    """A plan's bytes against the device memory that plans of it take: the footprint, and with passes on the
+    chip (no tile width forced) their mailboxes, tables and staging."""
+    import torch
+    from rtmuq2d_gb300 import workloads
+    p = workloads.params_tiny(nx=1201, nz=403, th=40, nt=400, time_slices=4).replace(**kw)
+    engine.Plan(p).close()                                 # what the process loads once
+    free = torch.cuda.mem_get_info()[0]
+    plans = [engine.Plan(p) for _ in range(3)]
+    taken = free - torch.cuda.mem_get_info()[0]
+    said = sum(plan.nbytes for plan in plans)
+    for plan in plans:
+        plan.close()
+    fp = engine.footprint_bytes(p)
+    assert (said == 3 * fp) == bool(kw.get("tile_x")) and said >= 3 * fp
+    # two allocations a plan, each rounded up to 2 MB pages
+    assert said <= taken + (2 << 20) and taken <= said + 3 * 2 * (2 << 20) + (2 << 20)
