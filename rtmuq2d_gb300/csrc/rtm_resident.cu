@@ -18,6 +18,8 @@
 // The arithmetic of a cell is the per-step kernels', in the same operand order (lap8, d1x_w, ...):
 // SRC/stencilDFM.c:17-29, SRC/absorbingBoundaryCondition.c:150-361, SRC/forward_modeling.c:98-130,
 // SRC/backward_modeling.c:268-297.
+#include <algorithm>
+
 #include "rtm_device.cuh"
 
 namespace rtm {
@@ -1624,21 +1626,29 @@ __global__ void __launch_bounds__(256) k_unpack16(const __grid_constant__ Pack16
     st4(out, q);
 }
 
-cudaError_t launch_pack16(int kind, bool pack, const Pack16 &a, int slots, cudaStream_t s)
+cudaError_t launch_pack16(int kind, bool pack, const Pack16 &all, int slots, cudaStream_t s)
 {
-    if (slots <= 0) return cudaSuccess;
-    const int groups = kind == kRingStrip ? strip_blocks_host(a.g) : a.g.tiles;
-    const dim3 grid(pack ? groups : (int)((a.slot_elems / 4 + 255) / 256), slots);
-    if (pack) {
-        if (kind == kRingTile) k_pack16<kRingTile><<<grid, 256, 0, s>>>(a);
-        else if (kind == kSnapTile) k_pack16<kSnapTile><<<grid, 256, 0, s>>>(a);
-        else k_pack16<kRingStrip><<<grid, 256, 0, s>>>(a);
-    } else {
-        if (kind == kRingTile) k_unpack16<kRingTile><<<grid, 256, 0, s>>>(a);
-        else if (kind == kSnapTile) k_unpack16<kSnapTile><<<grid, 256, 0, s>>>(a);
-        else k_unpack16<kRingStrip><<<grid, 256, 0, s>>>(a);
+    constexpr int kMost = 65535;                         // blocks of a grid's second dimension
+    const int groups = kind == kRingStrip ? strip_blocks_host(all.g) : all.g.tiles;
+    for (int k = 0; k < slots; k += kMost) {
+        Pack16 a = all;
+        a.stage += (size_t)k * a.slot_elems;
+        a.store = static_cast<unsigned char *>(a.store) + (size_t)k * a.slot_elems * 2;
+        a.scales += (size_t)k * a.scales_per_slot;
+        const dim3 grid(pack ? groups : (int)((a.slot_elems / 4 + 255) / 256), std::min(slots - k, kMost));
+        if (pack) {
+            if (kind == kRingTile) k_pack16<kRingTile><<<grid, 256, 0, s>>>(a);
+            else if (kind == kSnapTile) k_pack16<kSnapTile><<<grid, 256, 0, s>>>(a);
+            else k_pack16<kRingStrip><<<grid, 256, 0, s>>>(a);
+        } else {
+            if (kind == kRingTile) k_unpack16<kRingTile><<<grid, 256, 0, s>>>(a);
+            else if (kind == kSnapTile) k_unpack16<kSnapTile><<<grid, 256, 0, s>>>(a);
+            else k_unpack16<kRingStrip><<<grid, 256, 0, s>>>(a);
+        }
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 }  // namespace rtm

@@ -136,3 +136,14 @@ def test_plan_bytes_are_what_it_takes(engine, kw):
     assert (said == 3 * fp) == bool(kw.get("tile_x")) and said >= 3 * fp
     # two allocations a plan, each rounded up to 2 MB pages
     assert said <= taken + (2 << 20) and taken <= said + 3 * 2 * (2 << 20) + (2 << 20)
+
+
+def test_more_snapshots_than_a_grid_has_rows(engine):
+    """16-bit snapshots of more steps than the 65535 blocks of a launch's second dimension, staged at once."""
+    nt = 66000
+    p, vel, wav, seis = _request(engine, 1, 4, (12, 12, 12, 12), nt, 1, 3, storage=0, precision=2, rec_count=1,
+                                 shot_x=0, shot_z=1)
+    got = engine.migrate_shot(p, vel, wav, seis)
+    want = engine.migrate_shot(p.replace(tile_x=16), vel, wav, seis)
+    assert np.abs(want[0]).max() > 0
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
