@@ -968,14 +968,20 @@ static int run_forward(rtm_plan *P, const float *d_vel, int vel_pitch, const flo
     return RTM_OK;
 }
 
+// What the wait that set the status bits was for.
+static const char *waited_for(unsigned st)
+{
+    return st & ST_EXCHANGE_TIMEOUT ? "an exchange between the blocks of a resident pass" : "a tile load";
+}
+
 static int check_status(rtm_plan *P)
 {
     unsigned st = 0;
     RTM_CUDA(cudaMemcpyAsync(&st, P->base + P->L.status, sizeof st, cudaMemcpyDeviceToHost, P->stream));
     RTM_CUDA(cudaStreamSynchronize(P->stream));
-    if (st & ST_TMA_TIMEOUT) {
+    if (st) {
         cudaMemsetAsync(P->base + P->L.status, 0, sizeof st, P->stream);
-        return fail(RTM_ERR_TIMEOUT, "a tile load did not complete within its time limit");
+        return fail(RTM_ERR_TIMEOUT, "%s did not complete within its time limit", waited_for(st));
     }
     return RTM_OK;
 }
@@ -1725,7 +1731,7 @@ int rtm_stack_finish(rtm_stack *S, int normalize_by_self, float *stacked, float 
     S->d2h_bytes += (long long)b;
     unsigned st;
     memcpy(&st, S->h_pinned + 2 * n, sizeof st);
-    if (st & ST_TMA_TIMEOUT) return fail(RTM_ERR_TIMEOUT, "a tile load of a stacked shot did not complete within its time limit");
+    if (st) return fail(RTM_ERR_TIMEOUT, "%s of a stacked shot did not complete within its time limit", waited_for(st));
     memcpy(stacked, S->h_pinned, n * sizeof(float));
     memcpy(laplacian, S->h_pinned + n, n * sizeof(float));
     return RTM_OK;

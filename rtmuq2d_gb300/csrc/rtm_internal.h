@@ -38,7 +38,8 @@ enum : int {
 
 // Device-side error bits (StepArgs::status)
 enum : unsigned {
-    ST_TMA_TIMEOUT = 1u << 0,
+    ST_TMA_TIMEOUT = 1u << 0,          // a step kernel's tile load
+    ST_EXCHANGE_TIMEOUT = 1u << 1,     // a resident block's wait for a neighbour
 };
 
 struct Geom {

@@ -269,7 +269,7 @@ __device__ __forceinline__ bool res_recv(const ResBox &b, int tid, const unsigne
 #pragma unroll
         for (int k = 0; k < 2; ++k)
             if (have[k]) {
-                ok = x_poll<T>(x[k], p[k], tag, status) && ok;
+                ok = ok && x_poll<T>(x[k], p[k], tag, status);
                 T q[4];
                 x[k].get(q);
                 st4(tile + 4 * (in[r + k] & 0x7fffu), q);
@@ -1265,7 +1265,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if (t > t0) ok = res_recv<T>(box_in, tid, in, t >= 3 ? nin : nin0, tag, sm, status);
         if constexpr (NC == 0) tm_wait_st();
         if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicOr(status, ST_TMA_TIMEOUT);
+            if (tid == 0) atomicOr(status, ST_EXCHANGE_TIMEOUT);
             dead = true;
             break;
         }
@@ -1475,6 +1475,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             }
         }
     }
+    cp_async_wait_all();                                    // a block that gave up: the ring quads of its step
     if constexpr (NC == 0) {
         __syncthreads();
         if (tid < 32) tm_free(s_tm);

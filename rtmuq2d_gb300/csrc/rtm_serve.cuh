@@ -527,7 +527,7 @@ static int harvest(rtm_server *S, int m)
     S->slot_plan[m] = nullptr;
     S->slot_req[m] = nullptr;
     S->idle.push_back(P);
-    if (st) return fail(RTM_ERR_TIMEOUT, "a tile load of request %lld timed out", R->id);
+    if (st) return fail(RTM_ERR_TIMEOUT, "%s of request %lld did not complete within its time limit", waited_for(st), R->id);
     return RTM_OK;
 }
 
@@ -855,7 +855,7 @@ int rtm_server_step(rtm_server *S, int *n_active, int *n_queued)
         }
         unsigned flags[2] = {0, 0};
         RTM_CUDA(cudaMemcpy(flags, S->d_done, sizeof flags, cudaMemcpyDeviceToHost));
-        if (flags[1]) return fail(RTM_ERR_TIMEOUT, "a batched tile load timed out");
+        if (flags[1]) return fail(RTM_ERR_TIMEOUT, "%s of the server's members did not complete within its time limit", waited_for(flags[1]));
         for (int m = 0; m < S->max_members; ++m) {
             if (!S->slot_plan[m]) continue;
             if (S->res_pass[m] == 0) {
