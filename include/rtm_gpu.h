@@ -205,6 +205,14 @@ int rtm_autotune(const rtm_params *p, int steps, int *best_tile_x, float *ms_per
 /* ---- device-resident plan (inputs already in HBM) ------------------------------------ */
 typedef struct rtm_plan rtm_plan;
 
+/* A pass on the chip (tile_x = 0) is one cooperative launch that holds up to all SMs until it ends, and
+ * starts once they are free: work of other streams on the device runs before or after it, and a kernel of
+ * theirs that keeps an SM keeps the pass waiting.  Passes of several plans on several streams are ordered on
+ * the device so that those in flight fit the SMs; of grids that could do with half the chip each takes a part
+ * when others are in flight, and they run side by side with the same results.  Processes that share the
+ * device at the same time (MPS) are not ordered among one another: a pass whose blocks wait two seconds for
+ * one that has not started ends with RTM_ERR_TIMEOUT.  With tile_x set a pass runs step by step, between and
+ * beside other work. */
 int rtm_plan_create(const rtm_params *p, rtm_plan **plan);
 int rtm_plan_destroy(rtm_plan *plan);
 int rtm_plan_set_stream(rtm_plan *plan, void *stream);

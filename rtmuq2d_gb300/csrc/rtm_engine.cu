@@ -27,6 +27,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "rtm_gate.h"
 #include "rtm_gpu.h"
 #include "rtm_internal.h"
 #include "rtm_partition.h"
@@ -402,9 +403,16 @@ struct rtm_plan {
     struct Resident {
         int nctas = 0, cw = 0;
         size_t smem = 0;
+        double cost = 0.0;
         const void *jobs = nullptr;
         const rtm::ResCta *ctas = nullptr;
+        // fewer blocks, for passes beside other plans' (share of the chip -> blocks, empty when they do
+        // not fit): searched for at their first use; the device holds those of one share
+        std::map<int, rtm::ResPart> parts;
+        rtm::ResCta *part_ctas = nullptr;
+        int part_share = 0;
     } res[2];
+    bool res_shares = false;     // half the chip would do
     unsigned char *res_base = nullptr;
     size_t res_bytes = 0, xch_bytes = 0;
     unsigned long long *xch = nullptr;
@@ -748,7 +756,9 @@ static int resident_tables(rtm_plan *P, int sms)
                                : (int)std::max<size_t>(1, std::min<size_t>((size_t)P->L.nslots, (32u << 20) / slot));
         stage = slot * P->stage16_slots;
     }
-    const size_t total = 2 * jb + cb[0] + cb[1] + P->xch_bytes + stage;
+    P->res_shares = !part[0].ctas.empty() && !part[1].ctas.empty() && (double)P->g.dimx * P->g.dimz <= kResCells * (sms / 2);
+    const size_t pb = P->res_shares ? align_up((size_t)(sms / 2) * sizeof(ResCta), 256) : 0;
+    const size_t total = 2 * jb + cb[0] + cb[1] + P->xch_bytes + stage + 2 * pb;
     if (cudaMalloc(&P->res_base, total) != cudaSuccess) {      // no room: per-step kernels
         cudaGetLastError();
         P->res_base = nullptr;
@@ -768,9 +778,12 @@ static int resident_tables(rtm_plan *P, int sms)
         P->res[b].smem = part[b].smem;
         P->res[b].cw = part[b].cw;
         P->res[b].nctas = (int)part[b].ctas.size();
+        P->res[b].cost = part[b].cost;
     }
     P->xch = reinterpret_cast<unsigned long long *>(P->res_base + off);
     if (stage) P->stage16 = reinterpret_cast<float *>(P->res_base + off + P->xch_bytes);
+    for (int b = 0; pb && b < 2; ++b)
+        P->res[b].part_ctas = reinterpret_cast<ResCta *>(P->res_base + total - (size_t)(2 - b) * pb);
     RTM_CUDA(cudaMemcpyAsync(P->res_base, h.data(), h.size(), cudaMemcpyHostToDevice, P->stream));
     RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
     RTM_CUDA(cudaStreamSynchronize(P->stream));
@@ -802,28 +815,127 @@ static bool resident_now(rtm_plan *P, int back)
     return cs == cudaStreamCaptureStatusNone;
 }
 
-// Cooperative launches of one device run one after the other: each holds every SM it uses until
-// its last step, so two in flight could wait for SMs the other holds.  The later one's stream
-// waits for the earlier one's end on the device; the host waits for nothing.
+// The cooperative launches of each device (rtm_gate.h): the later one's stream waits for the ends of those
+// it must not run beside, on the device; the host waits for nothing.
 struct ResGate {
     std::mutex mu;
-    cudaEvent_t last[64] = {};
+    struct Device {
+        int sms = 0;
+        ResBook<cudaEvent_t> book;
+        std::vector<cudaEvent_t> spare;
+    } dev[64];
 };
 static ResGate g_gate;
 
-// One cooperative launch on `stream`, after every earlier one on the device.
-template <typename T>
-static int gated_resident(const ResLaunch<T> &L, cudaStream_t stream)
+// The current device's launches, those that have ended taken out where they matter to one on `stream`:
+// launches of other streams, or many of its own (g_gate.mu held).
+static int gate_open(cudaStream_t stream, ResGate::Device **out, unsigned long long *id)
 {
+    RTM_CUDA(cudaStreamGetId(stream, id));
     int dev = 0;
     RTM_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail(RTM_ERR_INVALID, "device ordinal %d out of range", dev);
+    ResGate::Device &D = g_gate.dev[dev];
+    if (!D.sms) RTM_CUDA(cudaDeviceGetAttribute(&D.sms, cudaDevAttrMultiProcessorCount, dev));
+    *out = &D;
+    const auto &open = D.book.open;
+    if (open.empty() || (open.size() == 1 && open[0].stream == *id && open[0].runs.size() < 8)) return RTM_OK;
+    // events may be asked while another stream is being captured
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RTM_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    D.book.prune([&](cudaEvent_t end) {
+        if (cudaEventQuery(end) == cudaSuccess) {
+            D.spare.push_back(end);
+            return true;
+        }
+        cudaGetLastError();
+        return false;
+    });
+    RTM_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    return RTM_OK;
+}
+
+// One cooperative launch on `stream`.
+template <typename T>
+static int gated_resident(const ResLaunch<T> &L, bool shares, cudaStream_t stream)
+{
     std::lock_guard<std::mutex> lk(g_gate.mu);
-    cudaEvent_t &ev = g_gate.last[dev];
-    if (!ev) RTM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    else RTM_CUDA(cudaStreamWaitEvent(stream, ev, 0));
+    ResGate::Device *D = nullptr;
+    unsigned long long id = 0;
+    RTM_TRY(gate_open(stream, &D, &id));
+    for (const auto &w : D->book.before(id, L.nctas, D->sms))
+        RTM_CUDA(cudaStreamWaitEvent(stream, D->book.open[w.first].runs[w.second].end, 0));
+    if (D->spare.empty()) {
+        cudaEvent_t e = nullptr;
+        RTM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        D->spare.push_back(e);
+    }
     RTM_CUDA(launch_resident<T>(L, stream));
-    RTM_CUDA(cudaEventRecord(ev, stream));
+    const cudaEvent_t end = D->book.launched(id, L.nctas, shares, [&] {
+        cudaEvent_t e = D->spare.back();
+        D->spare.pop_back();
+        return e;
+    });
+    RTM_CUDA(cudaEventRecord(end, stream));
+    return RTM_OK;
+}
+
+// Whether a plan's passes fit an s-th of the chip, both of them, and take less than s times as long there
+// as on the whole (of 2000 x 600 with rings only the forward pass fits half: sharing cost two plans 11.6 ms
+// a shot of 300 steps a pass, taking turns 9.4).
+static bool resident_fits_share(rtm_plan *P, int s, int sms)
+{
+    for (int back = 0; back < 2; ++back) {
+        auto &R = P->res[back];
+        auto it = R.parts.find(s);
+        if (it == R.parts.end()) {
+            const int fields = back && P->p.storage == RTM_STORE_RING ? 2 : 1;
+            ResPart part;
+            if (!res_partition(P->g, fields, (int)P->es, sms / s, part) || part.xch_quads * 8 * P->es > P->xch_bytes ||
+                part.cost >= s * R.cost)
+                part = ResPart();
+            it = R.parts.emplace(s, std::move(part)).first;
+        }
+        if (it->second.ctas.empty()) return false;
+    }
+    return true;
+}
+
+// The share of the chip that a pass takes, its blocks on the device: all of it (1), or beside n passes in
+// flight on other streams that could do with half, an (n + 1)th, rounded to one of a few shares, or the
+// smallest larger one that it fits.  Steady shots of n plans on n streams, ms a shot of all (step kernels;
+// whole chips in turn; shares): 8 of 96 x 64, 2000 steps a pass, 36.4, 71, 20.4; 8 of 400 x 200, 1000
+// steps, 29.6, 44, 19.1; 2 of 1200 x 400, 500 steps, 11.6, 12.0, 8.0.
+static int resident_share(rtm_plan *P, int back, int *share)
+{
+    *share = 1;
+    if (!P->res_shares) return RTM_OK;
+    int n = 1, sms = 0;
+    {
+        std::lock_guard<std::mutex> lk(g_gate.mu);
+        ResGate::Device *D = nullptr;
+        unsigned long long id = 0;
+        RTM_TRY(gate_open(P->stream, &D, &id));
+        n += D->book.sharers(id);
+        sms = D->sms;
+    }
+    if (n == 1) return RTM_OK;
+    static const int kShares[] = {2, 3, 4, 6, 8, 12, 16};
+    int k = 0;
+    while (k < 6 && kShares[k] < n) ++k;
+    while (k >= 0 && !resident_fits_share(P, kShares[k], sms)) --k;
+    if (k < 0) {
+        P->res_shares = false;
+        return RTM_OK;
+    }
+    auto &R = P->res[back];
+    const ResPart &part = R.parts.at(kShares[k]);
+    if (R.part_share != kShares[k]) {        // after the stream's last pass; the source has been read on return
+        R.part_share = 0;
+        RTM_CUDA(cudaMemcpyAsync(R.part_ctas, part.ctas.data(), part.ctas.size() * sizeof(ResCta), cudaMemcpyHostToDevice, P->stream));
+        R.part_share = kShares[k];
+    }
+    *share = kShares[k];
     return RTM_OK;
 }
 
@@ -835,6 +947,8 @@ static int run_resident(rtm_plan *P, int back, T *rec_out)
     const auto &R = P->res[back];
     const Geom &g = P->g;
     const int nt = g.nt;
+    int share = 1;
+    RTM_TRY(resident_share(P, back, &share));
     if (P->res_tag > 0xffffffffu - 4u * (unsigned)nt - 8u) {     // tags start over
         RTM_CUDA(cudaMemsetAsync(P->xch, 0, P->xch_bytes, P->stream));
         P->res_tag = 1;
@@ -853,6 +967,13 @@ static int run_resident(rtm_plan *P, int back, T *rec_out)
     L.nctas = R.nctas;
     L.cw = R.cw;
     L.smem = R.smem;
+    if (share > 1) {
+        const ResPart &part = R.parts.at(share);
+        L.ctas = R.part_ctas;
+        L.nctas = (int)part.ctas.size();
+        L.cw = part.cw;
+        L.smem = part.smem;
+    }
     L.xch = P->xch;
     L.rec_out = rec_out;
     L.status = P->at<unsigned>(P->L.status);
@@ -862,7 +983,7 @@ static int run_resident(rtm_plan *P, int back, T *rec_out)
         L.tag0 = P->res_tag;
         P->res_tag += (unsigned)(t1 - t0) + 2u;
         P->launches++;
-        return gated_resident<T>(L, P->stream);
+        return gated_resident<T>(L, P->res_shares, P->stream);
     };
     if (!P->stage16) {
         RTM_TRY(steps(0, nt));

@@ -391,7 +391,7 @@ static int step_resident(rtm_server *S, bool sampled)
         // one launch of a server step without batched members is timed, for rtm_server_kernel_ms
         const bool sample = w == 0 && sampled;
         if (sample) RTM_CUDA(cudaEventRecord(S->kev0, S->stream));
-        RTM_TRY(gated_resident<float>(L, S->stream));
+        RTM_TRY(gated_resident<float>(L, false, S->stream));
         if (sample) {
             RTM_CUDA(cudaEventRecord(S->kev1, S->stream));
             for (const Item &it : waves[w]) S->res_sampled = std::max(S->res_sampled, it.t1 - it.t0);
