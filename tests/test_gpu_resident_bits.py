@@ -95,3 +95,27 @@ def test_members_of_one_launch_equal_their_own(engine):
         want = engine.migrate_shot(*r)
         assert np.abs(want[0]).max() > 0
         assert np.array_equal(out[i][0], want[0]) and np.array_equal(out[i][1], want[1])
+
+
+@pytest.mark.parametrize("kw", ({}, dict(precision=1)))
+def test_resident_forward_with_an_adjoint_by_steps(engine, kw):
+    """3600 x 700 with rings: the forward pass fits the chip, the adjoint with its two fields does not."""
+    import torch
+    from rtmuq2d_gb300 import workloads
+    p = workloads.params_tiny(nx=3600, nz=700, th=50, nt=80, time_slices=4, n_wavelet=30).replace(**kw)
+    rng = np.random.default_rng(9)
+    ext = engine.extend_matrix(p, (1600 + 800 * rng.random((p.nx, p.nz))).astype(np.float32))
+    vel = torch.from_numpy(ext).cuda()
+    wav = torch.from_numpy(workloads.wavelet_for(p, 60.0)).cuda()
+    seis = torch.from_numpy((0.1 * rng.standard_normal((p.rec_count, p.nt))).astype(np.float32)).cuda()
+    plan = engine.Plan(p)
+    plan.forward(vel, wav)
+    forward = plan.launches
+    plan.adjoint(seis)
+    plan.sync()
+    assert forward < 12 and plan.launches - forward >= p.nt
+    plan.close()
+    _, a = _outputs(engine, torch, p, vel, wav, seis)
+    _, b = _outputs(engine, torch, p.replace(tile_x=16), vel, wav, seis)
+    for k, y in b.items():
+        assert np.abs(y).max() > 0 and np.array_equal(a[k], y), k
