@@ -4,9 +4,10 @@
 // A server holds up to kMaxMembers resident migrations ("members").  Requests are admitted
 // in arrival order while a member slot is free and their device footprint fits the HBM
 // budget; admission uploads the inputs and sets the member up (coef, seismogram transpose,
-// zeroed wavefields and image accumulators).  rtm_server_step replays a CUDA graph of
+// zeroed wavefields and image accumulators).  rtm_server_step launches the members' passes on the chip
+// (rtm_resident.cu, rtm_waves.h) and, for members that cannot run there, replays a CUDA graph of
 // `steps_per_launch` batched time steps (k_mstep + k_bpsi + k_bstrip per step, chained by
-// programmatic dependent launch): every active member advances one step per batched step,
+// programmatic dependent launch): each of those advances one step per batched step,
 // whatever its grid, time axis or pass.  Members that finished their backward pass are harvested (image
 // and self image copied to host buffers) and their slots freed for the next admissions --
 // continuous batching.  One thread drives a server; each server has its own stream.
@@ -410,7 +411,8 @@ static int step_resident(rtm_server *S, bool sampled)
 
 // Uploads one admitted request into slot m on the upload stream: the graph replaying on the
 // server's stream touches only active members, and this one becomes active (activate) after
-// the replay and these uploads.  The sources are the request's pageable host copies: each
+// the replay and these uploads.  (The copies overlap resident launches as well; the two small kernels get
+// the SMs that those leave over, or wait for their end.)  The sources are the request's pageable host copies: each
 // copy returns once its data is staged, so they are released right after.
 static int admit(rtm_server *S, int m, ServeRequest *R)
 {
@@ -500,7 +502,8 @@ static int activate(rtm_server *S)
 
 // A finished member's image and self image to its request, on the upload stream: the graph
 // replaying meanwhile skips the member (its state is past its backward pass), so the copies
-// overlap the replay.  The slot is free afterwards.
+// overlap the replay; beside resident launches, which hold most SMs, k_image_out and with it this
+// call mostly wait for their end.  The slot is free afterwards.
 static int harvest(rtm_server *S, int m)
 {
     NvtxRange range("rtm server harvest");
