@@ -147,3 +147,21 @@ def test_more_snapshots_than_a_grid_has_rows(engine):
     want = engine.migrate_shot(p.replace(tile_x=16), vel, wav, seis)
     assert np.abs(want[0]).max() > 0
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("steps_per_launch", (3, 16))
+def test_more_members_than_run_at_a_step(engine, steps_per_launch):
+    """Eleven members that fill the chip and six small ones: two or more of the waves run at a server step, and
+    every image equals the member's own."""
+    rs = [_request(engine, 2600, 600, (50, 50, 50, 50), 40, 4, k % 3, precision=0) for k in range(11)]
+    rs += [_request(engine, 96 + 7 * k, 64, (16, 16, 16, 16), 60 + 20 * k, 4, 20 + k, storage=k % 2) for k in range(6)]
+    srv = engine.Server(0, max_members=32, steps_per_launch=steps_per_launch)
+    ids = [srv.submit(*r) for r in rs]
+    out = srv.run_all()
+    srv.close()
+    want = {}
+    for k, r in enumerate(rs):
+        key = k % 3 if k < 11 else k
+        if key not in want:
+            want[key] = engine.migrate_shot(*r)
+        assert np.array_equal(out[ids[k]][0], want[key][0]) and np.array_equal(out[ids[k]][1], want[key][1]), k
